@@ -355,10 +355,10 @@ __global__ void __launch_bounds__(RB, (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 
             if (UOC)
             {
                 const float p0 = dead[a] ? 0.0f : alive[a] * euro[a];
-                fix_add(&paySlab[0], p0);
-                fix_add(&paySlab[2 * nPay], p0 * p0);
-                fix_add(&paySlab[2], euro[a]);
-                fix_add(&paySlab[2 * (nPay + 1)], euro[a] * euro[a]);
+                fix_add_s(&paySlab[0], p0);
+                fix_add_s(&paySlab[2 * nPay], p0 * p0);
+                fix_add_s(&paySlab[2], euro[a]);
+                fix_add_s(&paySlab[2 * (nPay + 1)], euro[a] * euro[a]);
                 agg = w0 * p0 + w1 * euro[a];
                 const float aEuro = dead[a] ? w1 : w0 * alive[a] + w1;
                 aAl = dead[a] ? 0.0f : w0 * euro[a];
@@ -373,13 +373,13 @@ __global__ void __launch_bounds__(RB, (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 
             }
             else
             {
-                fix_add(&paySlab[0], euro[a]);
-                fix_add(&paySlab[2 * nPay], euro[a] * euro[a]);
+                fix_add_s(&paySlab[0], euro[a]);
+                fix_add_s(&paySlab[2 * nPay], euro[a] * euro[a]);
                 agg = w0 * euro[a];
                 ax = euro[a] > 0.0f ? w0 * sT[a] : 0.0f;
             }
-            fix_add(&paySlab[2 * (2 * nPay)], agg);
-            fix_add(&paySlab[2 * (2 * nPay + 1)], agg * agg);
+            fix_add_s(&paySlab[2 * (2 * nPay)], agg);
+            fix_add_s(&paySlab[2 * (2 * nPay + 1)], agg * agg);
             live[a] = ax != 0.0f || aAl != 0.0f;
             if (live[a])
             {
@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(RB, (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 
                 const float S = es[(F_S + a) * rowStride + col];
                 ax += aAl * before * invTwo * S;
             }
-            fix_add(&slab[0], ax / spot);  // x_0 = log(spot)
+            fix_add_s(&slab[0], ax / spot);  // x_0 = log(spot)
         }
         head += n;
         __syncthreads();

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
     auto nodeAdd = [&](int idx, long long v) {
         constexpr long long LIM = 1LL << 50;
         if (!p.nodeDirect && v < LIM && v > -LIM)
-            atomicAdd(reinterpret_cast<unsigned long long*>(&node[idx]), (unsigned long long)v);
+            shared_add64(&node[idx], v);
         else
             node_flush(&p.acc[2 * (1 + idx)], v);
     };
@@ -318,8 +318,8 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
                     const Real pay = (m > Real(0) ? m : Real(0)) / N;
                     if (pay != Real(0))
                     {
-                        fix_add(&paySlab[2 * (payBase + k)], pay);
-                        fix_add(&paySlab[2 * (sqBase + k)], pay * pay);
+                        fix_add_s(&paySlab[2 * (payBase + k)], pay);
+                        fix_add_s(&paySlab[2 * (sqBase + k)], pay * pay);
                     }
                     if (po) po[(path0 + a) * nPay + k] = double(pay);
                     if (RISK) agg[a] += wts[k] * pay;
@@ -373,18 +373,18 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
             {
                 const Real m = fE[a] - strike;
                 const Real pay = (m > Real(0) ? m : Real(0)) * dE[a] / nE[a];
-                fix_add(&paySlab[2 * payBase], pay);
-                fix_add(&paySlab[2 * sqBase], pay * pay);
+                fix_add_s(&paySlab[2 * payBase], pay);
+                fix_add_s(&paySlab[2 * sqBase], pay * pay);
                 agg[a] = w0 * pay;
                 if (po) po[(path0 + a) * nPay] = double(pay);
             }
             else if (PROD == PROD_UOC)
             {
                 const Real p0 = dead[a] ? Real(0) : alive[a] * euro[a];
-                fix_add(&paySlab[2 * payBase], p0);
-                fix_add(&paySlab[2 * sqBase], p0 * p0);
-                fix_add(&paySlab[2 * (payBase + 1)], euro[a]);
-                fix_add(&paySlab[2 * (sqBase + 1)], euro[a] * euro[a]);
+                fix_add_s(&paySlab[2 * payBase], p0);
+                fix_add_s(&paySlab[2 * sqBase], p0 * p0);
+                fix_add_s(&paySlab[2 * (payBase + 1)], euro[a]);
+                fix_add_s(&paySlab[2 * (sqBase + 1)], euro[a] * euro[a]);
                 agg[a] = w0 * p0 + w1 * euro[a];
                 if (po)
                 {
@@ -394,15 +394,15 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
             }
             else if (PROD == PROD_CONTINGENT)
             {
-                fix_add(&paySlab[2 * payBase], cPay[a]);
-                fix_add(&paySlab[2 * sqBase], cPay[a] * cPay[a]);
+                fix_add_s(&paySlab[2 * payBase], cPay[a]);
+                fix_add_s(&paySlab[2 * sqBase], cPay[a] * cPay[a]);
                 agg[a] = w0 * cPay[a];
                 if (po) po[(path0 + a) * nPay] = double(cPay[a]);
             }
             if (RISK)
             {
-                fix_add(&paySlab[2 * aggBase], agg[a]);
-                fix_add(&paySlab[2 * (aggBase + 1)], agg[a] * agg[a]);
+                fix_add_s(&paySlab[2 * aggBase], agg[a]);
+                fix_add_s(&paySlab[2 * (aggBase + 1)], agg[a] * agg[a]);
             }
         }
         if (!RISK) return;
@@ -564,8 +564,8 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
                         const Real wa = cA[s], wb = cB[s];
                         auto put = [&](int j, Real aY) {
                             if (aY == Real(0)) return;
-                            fix_add(&node[2 * (j * nT + ca)], aY * wa);
-                            if (wb != Real(0)) fix_add(&node[2 * (j * nT + cb)], aY * wb);
+                            fix_add_s(&node[2 * (j * nT + ca)], aY * wa);
+                            if (wb != Real(0)) fix_add_s(&node[2 * (j * nT + cb)], aY * wb);
                         };
                         if (flat) put(k, av);
                         else
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
 #pragma unroll
             for (int a = 0; a < NP; ++a)
                 if (a < nAct) sp += ax[a];
-            fix_add(&slab[0], sp / spot);  // x_0 = log(spot)
+            fix_add_s(&slab[0], sp / spot);  // x_0 = log(spot)
         }
         else
         {
@@ -607,10 +607,10 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
                 s2 += aR[a];
                 s3 += aDv[a];
             }
-            fix_add(&slab[0], s0);
-            fix_add(&slab[2], s1);
-            fix_add(&slab[4], s2);
-            fix_add(&slab[6], s3);
+            fix_add_s(&slab[0], s0);
+            fix_add_s(&slab[2], s1);
+            fix_add_s(&slab[4], s2);
+            fix_add_s(&slab[6], s3);
         }
     };
 

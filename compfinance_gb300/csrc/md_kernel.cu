@@ -65,8 +65,27 @@ __host__ __device__ inline MdSmem md_smem(int rng, int fp32, const McParams& p)
     return S;
 }
 
+// v into a shared pair that every lane of a warp adds to.  The wide instances (NA > 4) hold up to
+// 150 of these sums and keep the shorter form of the split.
+template <int NA>
+__device__ __forceinline__ void md_add(long long* slot, float v) { fix_add_s(slot, v); }
+template <int NA>
+__device__ __forceinline__ void md_add(long long* slot, double v)
+{
+    if constexpr (NA <= 4)
+        fix_add_s(slot, v);
+    else
+    {
+        long long hi, lo;
+        fix_split_fp64(v, hi, lo);
+        shared_add64(slot, hi);
+        shared_add64(slot + 1, lo);
+    }
+}
+
+// FP64, up to four assets: five blocks per SM (four with mrg32k3a, which carries two paths)
 template <int RNGK, class Real, int NA>
-__global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
+__global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RNGK == RNG_SOBOL ? 5 : 4) md_kernel(const McParams p)
 {
     constexpr int NP = RNGK == RNG_MRG ? 2 : 1;
     constexpr bool F32 = std::is_same<Real, float>::value;
@@ -197,12 +216,12 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
                     {
                         const Real m = b - sK[k];
                         const Real v = (m > Real(0) ? m : Real(0)) / num;
-                        fix_add(&accPay[2 * k], v);
-                        fix_add(&accPay[2 * (nPay + k)], v * v);
+                        md_add<NA>(&accPay[2 * k], v);
+                        md_add<NA>(&accPay[2 * (nPay + k)], v * v);
                         agg += sW[k] * v;
                     }
-                    fix_add(&accPay[2 * (2 * nPay)], agg);
-                    fix_add(&accPay[2 * (2 * nPay + 1)], agg * agg);
+                    md_add<NA>(&accPay[2 * (2 * nPay)], agg);
+                    md_add<NA>(&accPay[2 * (2 * nPay + 1)], agg * agg);
                     continue;
                 }
                 // autocall (mcPrdMulti.h:368-416)
@@ -223,11 +242,11 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
                     pay[ap] += alive[ap] / num;
                     const Real m = kput - worst;
                     pay[ap] -= alive[ap] * (m > Real(0) ? m : Real(0)) / kput / num;
-                    fix_add(&accPay[0], pay[ap]);
-                    fix_add(&accPay[2 * nPay], pay[ap] * pay[ap]);
+                    md_add<NA>(&accPay[0], pay[ap]);
+                    md_add<NA>(&accPay[2 * nPay], pay[ap] * pay[ap]);
                     const Real agg = sW[0] * pay[ap];
-                    fix_add(&accPay[2 * (2 * nPay)], agg);
-                    fix_add(&accPay[2 * (2 * nPay + 1)], agg * agg);
+                    md_add<NA>(&accPay[2 * (2 * nPay)], agg);
+                    md_add<NA>(&accPay[2 * (2 * nPay + 1)], agg * agg);
                 }
             }
         }
@@ -273,7 +292,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
 #pragma unroll
                         for (int a = 0; a < NA; ++a)
                             if (a < nA) sb[a] += bb * sAsset[a];
-                        fix_add(&sAcc[2 * (L.num + e)], nb);
+                        md_add<NA>(&sAcc[2 * (L.num + e)], nb);
                     }
                     else
                     {
@@ -299,7 +318,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
                             aliveBar = w0 * (cpn * dtc + Real(1) - f) / num + aliveBar * f;
                             worstBar = inside ? -fBar / Real(2) / sm : Real(0);
                         }
-                        fix_add(&sAcc[2 * (L.num + e)], -w0 * payE / num);
+                        md_add<NA>(&sAcc[2 * (L.num + e)], -w0 * payE / num);
 #pragma unroll
                         for (int a = 0; a < NA; ++a)
                             if (a == wi) sb[a] += worstBar / sAsset[a];
@@ -327,7 +346,7 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
                     if (dy == MD_NORMAL)
                     {
                         fwdBar = abar;
-                        fix_add(&sAcc[2 * (L.std_ + i * nA + a)], abar * cw);
+                        md_add<NA>(&sAcc[2 * (L.std_ + i * nA + a)], abar * cw);
                         cwBar = abar * sd;
                     }
                     else
@@ -338,11 +357,11 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
                         fwdBar = abar * E;
                         if (dy == MD_SURNORMAL) ab[a] += abar * (E - Real(1));
                         if (dy == MD_SUBNORMAL) ab[a] += abar * (Real(1) - E);
-                        fix_add(&sAcc[2 * (L.drift + i * nA + a)], ub);
-                        fix_add(&sAcc[2 * (L.std_ + i * nA + a)], ub * cw);
+                        md_add<NA>(&sAcc[2 * (L.drift + i * nA + a)], ub);
+                        md_add<NA>(&sAcc[2 * (L.std_ + i * nA + a)], ub * cw);
                         cwBar = ub * sd;
                     }
-                    fix_add(&sAcc[2 * (L.ff + i * nA + a)], fwdBar * sPrev);
+                    md_add<NA>(&sAcc[2 * (L.ff + i * nA + a)], fwdBar * sPrev);
                     sb[a] = fwdBar * ff;
 #pragma unroll
                     for (int b = 0; b <= a; ++b) lb[a * (a + 1) / 2 + b] += cwBar * wv[b];
@@ -352,12 +371,12 @@ __global__ void __launch_bounds__(MD_BLOCK) md_kernel(const McParams p)
             for (int a = 0; a < NA; ++a)
                 if (a < nA)
                 {
-                    fix_add(&sAcc[2 * (L.s0 + a)], sb[a]);
-                    if (ab[a] != Real(0)) fix_add(&sAcc[2 * (L.alpha + a)], ab[a]);
+                    md_add<NA>(&sAcc[2 * (L.s0 + a)], sb[a]);
+                    if (ab[a] != Real(0)) md_add<NA>(&sAcc[2 * (L.alpha + a)], ab[a]);
 #pragma unroll
                     for (int b = 0; b <= a; ++b)
                         if (lb[a * (a + 1) / 2 + b] != Real(0))
-                            fix_add(&sAcc[2 * (L.chol + a * nA + b)], lb[a * (a + 1) / 2 + b]);
+                            md_add<NA>(&sAcc[2 * (L.chol + a * nA + b)], lb[a * (a + 1) / 2 + b]);
                 }
         }
     };

@@ -191,17 +191,17 @@ __global__ void __launch_bounds__(MC_BLOCK) multi_kernel(const MultiParams mp)
                 const int m = bucketOf(e, F);
                 const int bk = mp.evOff[e] + m;
                 const Real iN = Real(1) / N;
-                fix_add(&sVal[2 * (5 * bk + 0)], iN);
-                fix_add(&sVal[2 * (5 * bk + 1)], F * iN);
-                fix_add(&sVal[2 * (5 * bk + 2)], iN * iN);
-                fix_add(&sVal[2 * (5 * bk + 3)], F * iN * iN);
-                fix_add(&sVal[2 * (5 * bk + 4)], F * F * iN * iN);
+                fix_add_s(&sVal[2 * (5 * bk + 0)], iN);
+                fix_add_s(&sVal[2 * (5 * bk + 1)], F * iN);
+                fix_add_s(&sVal[2 * (5 * bk + 2)], iN * iN);
+                fix_add_s(&sVal[2 * (5 * bk + 3)], F * iN * iN);
+                fix_add_s(&sVal[2 * (5 * bk + 4)], F * F * iN * iN);
                 if (MODEL == MODEL_BS && m > 0)
                 {
                     for (int q = 0; q < 4; ++q)
                     {
-                        fix_add(&sBs[2 * (8 * bk + 2 * q)], F * iN * (dlnF[q] - dlnN[q]));  // a
-                        fix_add(&sBs[2 * (8 * bk + 2 * q + 1)], -iN * dlnN[q]);              // b
+                        fix_add_s(&sBs[2 * (8 * bk + 2 * q)], F * iN * (dlnF[q] - dlnN[q]));  // a
+                        fix_add_s(&sBs[2 * (8 * bk + 2 * q + 1)], -iN * dlnN[q]);              // b
                     }
                 }
                 if (MODEL == MODEL_DUPIRE)

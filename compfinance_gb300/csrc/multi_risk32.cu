@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(MB) multi32_forward(const Multi32Args A)
         if (lo > 0)
         {
             const int bk = sEvOff[e] + lo;
-            fix_add(sVal + 2 * bk, S);
+            fix_add_s(sVal + 2 * bk, S);
             atomicAdd(hist + bk, 1);
         }
     };
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(MB) multi32_reverse(const Multi32Args A)
                     cur = nxt;
                 }
             }
-            fix_add(spotSlab, ax / spot);  // x_0 = log(spot)
+            fix_add_s(spotSlab, ax / spot);  // x_0 = log(spot)
         }
         __syncthreads();
         // the chunk's slab -> the bucket's row (node words in units of 2^-nodeShiftF: exact in hi)

@@ -1,0 +1,14 @@
+"""Host check of the fixed-point arithmetic shared with the kernels (no GPU): tests/cpp/fixed_test.cpp."""
+import os
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def test_fixed_point(tmp_path):
+    exe = str(tmp_path / "fixed_test")
+    csrc = os.path.join(ROOT, "compfinance_gb300", "csrc")
+    subprocess.check_call(["g++", "-std=c++17", "-O2", "-I", csrc, os.path.join(ROOT, "tests", "cpp", "fixed_test.cpp"),
+                           "-o", exe])
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and all(x.startswith("ok") for x in r.stdout.splitlines()), r.stdout + r.stderr

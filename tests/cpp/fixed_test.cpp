@@ -3,6 +3,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <random>
 
 #include "fixed64.h"
@@ -42,7 +43,7 @@ int main()
             check(v);
             check(-v);
         }
-    for (double v : {0.0, -0.0, INFINITY, -INFINITY, std::ldexp(1.0, 42), std::nextafter(std::ldexp(1.0, 42), 0.0),
+    for (const double v : std::initializer_list<double>{0.0, -0.0, (double)INFINITY, -(double)INFINITY, std::ldexp(1.0, 42), std::nextafter(std::ldexp(1.0, 42), 0.0),
                      std::ldexp(1.0, -61), std::ldexp(3.0, -61), std::ldexp(1.0, -62), 5e-324})
     {
         check(v);

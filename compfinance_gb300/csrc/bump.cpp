@@ -40,7 +40,7 @@ int bump_risk_reprice(Context& c, const std::string& mid, const std::string& pid
     n64.precision = CF_FP64;
     const int nPay = base->nPay, nParam = base->nParam;
     std::vector<double> v0(nPay), vb(nPay);
-    if ((rc = c.enqueue(*base, n64, false, nullptr)) || (rc = c.fetch(v0.data(), nullptr, nullptr, nullptr))) return rc;
+    if ((rc = c.enqueue(*base, n64, false, nullptr, nullptr, true)) || (rc = c.fetch(v0.data(), nullptr, nullptr, nullptr))) return rc;
     if (values) std::memcpy(values, v0.data(), size_t(nPay) * 8);
     const ModelDesc& m0 = c.models.at(mid);
     const ProductDesc& pd = c.products.at(pid);
@@ -52,7 +52,7 @@ int bump_risk_reprice(Context& c, const std::string& mid, const std::string& pid
         x += kBump;
         Plan bp;
         if ((rc = c.buildPlan(mb, pd, bp))) return rc;
-        if ((rc = c.enqueue(bp, n64, false, nullptr)) || (rc = c.fetch(vb.data(), nullptr, nullptr, nullptr)))
+        if ((rc = c.enqueue(bp, n64, false, nullptr, nullptr, true)) || (rc = c.fetch(vb.data(), nullptr, nullptr, nullptr)))
             return rc;
         x = keep;
         for (int k = 0; k < nPay; ++k) risks[size_t(i) * nPay + k] = 1.0e+08 * (vb[k] - v0[k]);

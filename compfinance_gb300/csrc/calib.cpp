@@ -326,7 +326,7 @@ int cf_dupire_superbucket_bump(cf_context* ctx, const cf_ivs* ivs, double spot, 
         int e = c.getPlan(mid, productId, plan);
         if (e) return e;
         std::vector<double> v(plan->nPay);
-        if ((e = c.enqueue(*plan, n64, false, nullptr)) || (e = c.fetch(v.data(), nullptr, nullptr, nullptr))) return e;
+        if ((e = c.enqueue(*plan, n64, false, nullptr, nullptr, true)) || (e = c.fetch(v.data(), nullptr, nullptr, nullptr))) return e;
         out = 0.0;
         for (int k = 0; k < plan->nPay; ++k) out += notionals[k] * v[k];  // inner_product in payoff order
         return CF_OK;

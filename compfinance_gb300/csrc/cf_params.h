@@ -8,6 +8,8 @@
 
 #include <cstdint>
 
+#include "fixed64.h"
+
 namespace cf {
 
 enum ModelKind : int { MODEL_BS = 0, MODEL_DUPIRE = 1, MODEL_MULTI = 2 };
@@ -75,6 +77,34 @@ constexpr int NODE_SHIFT = ROW_SHIFT + WEIGHT_SHIFT;
 //   [nRisk, nRisk+nPay)          sum of payoff k
 //   [nRisk+nPay, nRisk+2nPay)    sum of payoff k squared
 //   nRisk+2nPay, +1              sum / sum of squares of the aggregate sum_k w_k payoff_k
+
+// The FP64 form's Dupire tables in fixed point (fixed64.h), for dupire_fx64.
+struct FxParams
+{
+    int r;                // bits of range taken from the fractions of the state and the vols
+    int sh;               // shift of the state that fills 63 bits over the grid
+    long long center;     // middle of the grid
+    long long half, grid;  // rounding of a step (fx_step)
+    int nBuckets, shift;  // buckets are 2^(32 + shift) state units wide, the first at x0h 2^32
+    int x0h;
+    const long long* bucket;
+    const FxInterval* interval;  // [nS + 1], for the reverse's weights
+    const long long* inv;        // [nS + 1] 2^123 / (interval's width 2^sh): weights in units of 2^-59
+    const FxVol* vol;            // [nSteps][nS + 1]
+    const double* slope;         // [nSteps][nS + 1] d vol / d y 2^-59
+    const FxStep* step;          // [nSteps]
+    // barrier smoothing band: y above yTop knocks out, above yBand survives by a factor linear in the
+    // spot; bandScale > 0: the factor is bandScale times fx_one_minus_exp8(yTop - y)
+    long long yTop, yBand;
+    double bandScale;
+    // inverse normal: pieces of the generator's lower and upper halves
+    const FxgPiece* g[2];
+    unsigned brk[2];
+    // risk launches: vol adjoints below 2^(53 - 60 + nodeShift) go to the shared slab, larger ones
+    // straight to the accumulators
+    int nodeShift;
+};
+
 struct McParams
 {
     // sizes: the launch simulates paths [firstPath, firstPath + nPath) of the run's sequence
@@ -191,6 +221,8 @@ struct McParams
     unsigned long long* claim;
     long long roundCap;
 
+    FxParams fx;
+
     // multi-asset displaced model (mcMdlMultiDisplaced.h) with Baskets / Autocall
     // (mcPrdMulti.h); nSteps is the number of time steps, the Gaussians per path nSteps * nA
     int nA;
@@ -217,7 +249,8 @@ struct McLaunch
     int grid, block;
     size_t smem;
     int fast;             // FP32 Dupire risk through dupire_risk32: 1 (rows read through L1) or 2
-                          // (rows staged by bulk copies, p.rowChunk > 0)
+                          // (rows staged by bulk copies, p.rowChunk > 0); 3: FP64 Dupire value or
+                          // risk through dupire_fx64 (block threads: 128 or 384)
 };
 
 int launch_mc(const McLaunch& l, const McParams& p, void* stream);   // returns cudaError_t
@@ -236,7 +269,7 @@ long long mc_rounds(const McLaunch& l, long long nPath, long long threads);
 // Reverse-sweep scratch fields of a risk launch of `rounds` unit rounds.
 int mc_scratch_fields(const McLaunch& l, long long rounds);
 // Bytes of a risk launch's scratch buffer: p.scratchFields fields [field][point][thread] for
-// grid*128 threads, then (dupire_risk32) one int64 node slab per block.  Sets p.nodeSlabOffset.
+// the grid's threads, then (dupire_risk32) one int64 node slab per block.  Sets p.nodeSlabOffset.
 size_t mc_scratch_bytes(const McLaunch& l, McParams& p, long long grid);
 // Whether a (model, product, precision, mode) launch of this plan runs dupire_risk32
 // (CF_FAST32=0 in the environment selects the generic kernel instead).

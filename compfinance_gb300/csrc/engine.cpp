@@ -28,6 +28,8 @@ int launch_mrg_state(const unsigned* A, const unsigned* B, unsigned s1, unsigned
 int launch_gauss(int sobol, int uniform, const unsigned* dir, const unsigned* A, const unsigned* B,
                  unsigned s1, unsigned s2, int dim, long long first, int n, double* out, void* stream);
 
+int fx_node_shift(const Plan& plan, int block);  // fx_plan.cpp
+
 thread_local std::string g_lastError;
 
 int fail(int code, const std::string& msg)
@@ -604,9 +606,28 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
             oTd = pk.vec(tdv);
             oBf = pk.vec(bf);
         }
+        // a European's or barrier's last date is maturity, and a European has no other
+        bool endOk = evAtStep[n] == plan.nEv - 1;
+        if (pd.kind == PROD_EUROPEAN)
+            for (int i = 0; i < n; ++i) endOk = endOk && evAtStep[i] < 0;
+        if ((pd.kind == PROD_UOC || pd.kind == PROD_EUROPEAN) && endOk)
+        {
+            plan.fxState = 0;
+            FxInput& in = plan.fxIn;
+            in.nSteps = n;
+            in.x0 = x0;
+            in.X.resize(nS);
+            for (int j = 0; j < nS; ++j) in.X[j] = X[j] - x0;
+            plan.fxTouch = sMax;
+            in.sq = std::move(sqv);
+            in.tw = std::move(twv);
+            in.colA = std::move(colA);
+            in.colB = std::move(colB);
+        }
         plan.nSteps = n;
         plan.yBytesD = Y.size() * 8;
         plan.yBytesF = Y.size() * 4;
+        if (plan.fxState == 0) plan.fxIn.Y = std::move(Y);
     }
     P.nSteps = plan.nSteps;
     plan.timeline = tl;
@@ -620,6 +641,8 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
         P.minusSmooth = pd.barrier - smooth;
         const double lb = P.minusSmooth > 0 ? std::log(P.minusSmooth) : -INFINITY;
         P.logBandD = lb - 1e-9;
+        plan.fxTop = P.barSmooth > 0 ? std::log(P.barSmooth) - P.x0d : -INFINITY;
+        plan.fxBand = lb - P.x0d;
         P.logBandF = float(m.kind == MODEL_DUPIRE ? lb - P.x0d - 1e-5 : lb - 1e-5);
     }
 
@@ -769,6 +792,7 @@ int Context::getPlan(const std::string& mid, const std::string& pid, Plan*& out)
         // once no kernel can still read them (a device-wide wait, as freeing them would be)
         CF_CUDA(cudaDeviceSynchronize());
         plan->tables.swap(it->second->tables);
+        plan->fxTables.swap(it->second->fxTables);
     }
     int rc = buildPlan(mi->second, pi->second, *plan);
     if (rc) return rc;
@@ -784,7 +808,7 @@ int Context::getPlan(const std::string& mid, const std::string& pid, Plan*& out)
 // into the slot's pinned buffer are all asynchronous on the slot's stream; slot.done is
 // recorded after them.
 int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk, const double* weights,
-                     long long firstPath, double* pathOut, long long chunkPaths, int maxBlocksPerSM)
+                     long long firstPath, double* pathOut, long long chunkPaths, int maxBlocksPerSM, bool generic)
 {
     if (num.numPath <= 0) return fail(CF_E_ARG, "numPath must be positive");
     if (firstPath < 0 || firstPath % 64) return fail(CF_E_ARG, "firstPath must be a non-negative multiple of 64");
@@ -843,7 +867,50 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     size_t smem0 = 0, smem1 = 0;
     int occ0 = 0, occ1 = 0;
     l.fast = mc_use_fast32(plan.base, plan.prod, l.fp32, l.risk);
-    if (l.fast)
+    l.block = 128;
+    // FP64 Dupire European and barrier runs in fixed point at every size their tables fit: 60x30 weekly
+    // barrier risk 9.5 -> 0.62 ms at 2^18 paths (141 -> 5.6 ms at 2^22), its value 5.2 -> 0.30 ms,
+    // 20x10 grid and 10^5 x 52 steps 0.85 -> 0.14 ms against the generic kernel
+    if (!fp32 && !generic && fxReady(plan) && fxGauss(sobol))
+    {
+        p.fx = plan.fx;
+        const int g0 = sobol ? FXG_SOBOL_LOWER : FXG_MRG, g1 = sobol ? FXG_SOBOL_UPPER : FXG_MRG;
+        p.fx.g[0] = static_cast<const FxgPiece*>(fxg[sobol ? 1 : 0].ptr);
+        p.fx.g[1] = p.fx.g[0] + (sobol ? FXG_PIECES : 0);
+        p.fx.brk[0] = fxgBrk[g0];
+        p.fx.brk[1] = fxgBrk[g1];
+        l.fast = 3;
+        // a node slab of many nodes is shared by a larger block when that keeps more threads resident
+        int best = 0, block = 128;
+        for (int b : {128, 384})
+        {
+            if (b > 128 && !risk) break;
+            l.block = b;
+            size_t n = 0;
+            int occ = 0;
+            mc_smem_bytes(l, p, 0, &n);
+            if (n > 227 * 1024 || mc_occupancy(l, n, &occ)) continue;
+            if (occ * b > best)
+            {
+                best = occ * b;
+                block = b;
+            }
+        }
+        if (best)
+        {
+            l.block = block;
+            mc_smem_bytes(l, p, 0, &smem0);
+            rc = mc_occupancy(l, smem0, &occ0);
+            if (rc) return cuda_fail(cudaError_t(rc), "occupancy");
+            p.fx.nodeShift = fx_node_shift(plan, l.block);
+        }
+        else
+        {
+            l.fast = 0;
+            l.block = 128;
+        }
+    }
+    if (l.fast == 1)
     {
         // the local-vol rows (bulk copies) and the inverse-normal table go to shared memory when
         // that costs no occupancy
@@ -882,26 +949,28 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     // the whole run
     p.nPath = chunk;
     const long long threadsNeeded = sobol ? (p.nPath / 32 + 1) * 32 : (p.nPath + 1) / 2;
-    long long grid = (threadsNeeded + 127) / 128;
+    long long grid = (threadsNeeded + l.block - 1) / l.block;
     const long long maxGrid = (long long)numSMs * (maxBlocksPerSM > 0 ? std::min(occ, maxBlocksPerSM) : occ);
     if (grid > maxGrid) grid = maxGrid;
     if (grid < 1) grid = 1;
     l.grid = int(grid);
-    l.block = 128;
     if (risk)
     {
         // kernels index the scratch with 32-bit offsets: keep fields*(steps+1)*threads < 2^31
         // (sized for the full ring, the most fields a launch can need)
         const long long perThread = (long long)mc_scratch_fields(l, R32_RING) * (plan.nSteps + 1);
         const long long maxThreads = ((1LL << 31) - 1) / perThread;
-        if (grid * 128 > maxThreads) grid = std::max(1LL, maxThreads / 128);
+        if (grid * l.block > maxThreads) grid = std::max(1LL, maxThreads / l.block);
         l.grid = int(grid);
-        p.scratchThreads = grid * 128;
-        const long long rounds = mc_rounds(l, p.nPath, grid * 128);
+        p.scratchThreads = grid * l.block;
+        const long long rounds = mc_rounds(l, p.nPath, grid * l.block);
         p.scratchFields = mc_scratch_fields(l, rounds);
         p.roundCap = rounds < R32_RING ? rounds : 0;
         const size_t bytes = mc_scratch_bytes(l, p, grid);
-        if ((rc = slot.scratch.ensure(bytes, st))) return rc;
+        rc = slot.scratch.ensure(bytes, st);
+        if (rc == CF_E_NOMEM && l.fast == 3)  // the generic kernel's scratch is a third of it
+            return enqueue(slot, plan, num, risk, weights, firstPath, pathOut, chunkPaths, maxBlocksPerSM, true);
+        if (rc) return rc;
         p.scratch = slot.scratch.ptr;
     }
     int nLaunch = 0;
@@ -931,7 +1000,7 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
 
 // Estimated device footprint of a run (scratch of the reverse sweep + accumulators), the
 // admission currency of the serving loop.
-size_t Context::footprint(const Plan& plan, const cf_num_param& num, bool risk) const
+size_t Context::footprint(const Plan& plan, const cf_num_param& num, bool risk, bool generic) const
 {
     const bool sobol = num.useSobol != 0, fp32 = num.precision == CF_FP32;
     const int NP = sobol ? 1 : 2;
@@ -969,6 +1038,13 @@ size_t Context::footprint(const Plan& plan, const cf_num_param& num, bool risk) 
     }
     const int fields = plan.prod == PROD_EUROPEANS ? 1 + 3 * NP : mc_scratch_fields(l, mc_rounds(l, num.numPath, threads));
     size_t b = size_t(plan.nParam + 2 * plan.nPay + 2) * 16 + size_t(plan.nPay) * 12 + 4096;
+    if (risk && !fp32 && !generic && plan.fxState >= 0)
+    {
+        // dupire_fx64: at most 7 blocks of 128 or 2 of 384 threads per SM, a ring of round slots
+        l.fast = 3;
+        const long long t = std::min<long long>(needed + 383, (long long)numSMs * 7 * 128);
+        return b + size_t(mc_scratch_fields(l, mc_rounds(l, num.numPath, t))) * size_t(plan.nSteps + 1) * size_t(t) * 8;
+    }
     if (risk) b += size_t(fields) * size_t(plan.nSteps + 1) * size_t(threads) * (fp32 ? 4 : 8);
     if (risk && l.fast) b += size_t((threads + 127) / 128) * size_t(plan.base.nS) * size_t(plan.base.nT) * 8 + 256;
     // multi: bucket accumulators plus the finished per-payoff risks

@@ -12,6 +12,7 @@
 
 #include "../../include/cfgpu.h"
 #include "cf_params.h"
+#include "fx_tables.h"
 
 namespace cf {
 
@@ -114,6 +115,15 @@ struct Plan : std::enable_shared_from_this<Plan>
     std::vector<int> evAtStep;
     DevBuf tables;
     McParams base;
+    // FP64 Dupire runs in fixed point (dupire_fx64): what its tables are made from, kept until the
+    // first such run builds them (fxState: 0 not yet, 1 built into fxTables and fx, -1 the generic
+    // kernel runs: other products, or magnitudes beyond the fixed-point ranges)
+    int fxState = -1;
+    DevBuf fxTables;
+    FxParams fx;
+    FxInput fxIn;
+    int fxTouch = 0;  // most steps that share a time column
+    double fxTop = 0, fxBand = 0;  // fxTop, fxBand: log of the band's ends over S0
     // multi-asset model: derived quantities (md_layout) and their Jacobian to the model
     // parameters, [total][nParam], from the host-side adjoint of the model's initialisation
     std::vector<double> mdDerived, mdJac;
@@ -177,6 +187,8 @@ struct Context
     DevBuf invn;  // piecewise-cubic inverse normal tables of the FP32 kernels: mrg32k3a, Sobol
     const float* invnMrg = nullptr;
     const float* invnSobol = nullptr;
+    DevBuf fxg[2];  // fixed-point inverse normal of mrg32k3a and of Sobol's two halves (fx_plan.cpp)
+    unsigned fxgBrk[3] = {0, 0, 0};
     Slot main;
     unsigned long long h2d = 0, d2h = 0;  // cumulative transfer bytes
 
@@ -193,13 +205,18 @@ struct Context
     // consecutive path ranges of at most that many paths, each adding into the same exact
     // accumulators (bit-identical results), so that kernels of other streams get the device
     // between them.  maxBlocksPerSM > 0 caps the launch's resident blocks per SM below the
-    // kernel's occupancy, leaving room on every SM for kernels of other streams.
+    // kernel's occupancy, leaving room on every SM for kernels of other streams.  generic: FP64
+    // Dupire runs in double arithmetic (finite differences by bumping, runs that must fit the
+    // smaller scratch).
     int enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk, const double* weights,
                 long long firstPath = 0, double* pathOut = nullptr, long long chunkPaths = 0,
-                int maxBlocksPerSM = 0);
+                int maxBlocksPerSM = 0, bool generic = false);
+    // fx_plan.cpp: the fixed-point tables of a plan and of a generator, built on first use
+    bool fxReady(Plan& plan);
+    bool fxGauss(bool sobol);
     int fetch(Slot& slot, double* values, double* stderrs, double* aggregate, double* risks);
     bool ready(Slot& slot) const;
-    size_t footprint(const Plan& plan, const cf_num_param& num, bool risk) const;
+    size_t footprint(const Plan& plan, const cf_num_param& num, bool risk, bool generic = false) const;
     // AADriskMulti: the multi kernel (European portfolios) is asynchronous like enqueue
     bool multiFast(const Plan& plan) const;
     bool multi32Use(const Plan& plan, const cf_num_param& num) const;  // FP32 Dupire: multi_risk32.cu
@@ -213,10 +230,11 @@ struct Context
                       double* risks);
     int riskMulti(Plan& plan, const cf_num_param& num, double* values, double* risks);
     // main-slot conveniences of the synchronous API
-    int enqueue(Plan& plan, const cf_num_param& num, bool risk, const double* weights, double* pathOut = nullptr)
+    int enqueue(Plan& plan, const cf_num_param& num, bool risk, const double* weights, double* pathOut = nullptr,
+                bool generic = false)
     {
         main.stream = stream;
-        return enqueue(main, plan, num, risk, weights, 0, pathOut);
+        return enqueue(main, plan, num, risk, weights, 0, pathOut, 0, 0, generic);
     }
     int fetch(double* values, double* stderrs, double* aggregate, double* risks)
     {

@@ -1,0 +1,92 @@
+// Device tables of the FP64 Dupire kernel's fixed-point form (fx_tables.h, mc_dupire_fx64.cuh), built on
+// the first FP64 value or risk run of a (model, product) pair.
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "engine.h"
+#include "host_math.h"
+
+namespace cf {
+
+// The inverse normal's pieces of a generator (20 ms of host work per table), on first use; Sobol's two
+// halves have a table each.
+bool Context::fxGauss(bool sobol)
+{
+    DevBuf& buf = fxg[sobol ? 1 : 0];
+    if (buf.ptr) return true;
+    const int first = sobol ? FXG_SOBOL_LOWER : FXG_MRG, n = sobol ? 2 : 1;
+    std::vector<FxgPiece> g(size_t(n) * FXG_PIECES);
+    bool ok = true;
+    for (int k = 0; k < n; ++k)
+        ok = (fxgBrk[first + k] = inv_normal_table64(first + k, &g[size_t(k) * FXG_PIECES])) != 0 && ok;
+    const size_t bytes = g.size() * sizeof(FxgPiece);
+    ok = ok && buf.ensure(bytes) == CF_OK && cudaMemcpy(buf.ptr, g.data(), bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    if (!ok) buf.release();
+    return ok;
+}
+
+bool Context::fxReady(Plan& plan)
+{
+    if (plan.fxState != 0) return plan.fxState > 0;
+    FxHost h;
+    bool ok = fx_lower(plan.fxIn, h);
+    if (ok)
+    {
+        std::vector<unsigned char> buf;
+        auto put = [&](const void* src, size_t n) {
+            const size_t off = (buf.size() + 255) & ~size_t(255);
+            buf.resize(off + n);
+            std::memcpy(buf.data() + off, src, n);
+            return off;
+        };
+        auto vec = [&](const auto& v) { return put(v.data(), v.size() * sizeof(v[0])); };
+        const size_t oB = vec(h.bucket), oI = vec(h.interval), oN = vec(h.inv), oV = vec(h.vol), oS = vec(h.slope),
+                     oT = vec(h.step);
+        // the upload completes here: kernels on any slot's stream read the tables
+        ok = plan.fxTables.ensure(buf.size()) == CF_OK &&
+             cudaMemcpyAsync(plan.fxTables.ptr, buf.data(), buf.size(), cudaMemcpyHostToDevice, stream) == cudaSuccess &&
+             cudaStreamSynchronize(stream) == cudaSuccess;
+        h2d += buf.size();
+        const char* d = static_cast<const char*>(plan.fxTables.ptr);
+        FxParams& f = plan.fx;
+        std::memset(&f, 0, sizeof(f));
+        f.r = h.r;
+        f.sh = h.sh;
+        f.center = h.center;
+        f.grid = h.grid;
+        f.half = h.grid << 31;
+        f.nBuckets = int(h.bucket.size());
+        f.shift = h.shift;
+        f.x0h = h.x0h;
+        f.bucket = reinterpret_cast<const long long*>(d + oB);
+        f.interval = reinterpret_cast<const FxInterval*>(d + oI);
+        f.inv = reinterpret_cast<const long long*>(d + oN);
+        f.vol = reinterpret_cast<const FxVol*>(d + oV);
+        f.slope = reinterpret_cast<const double*>(d + oS);
+        f.step = reinterpret_cast<const FxStep*>(d + oT);
+        auto state = [&](double x) {  // the last state not above x
+            const double v = std::floor(std::ldexp(x, FX_Y - h.r));
+            return !(v > -9.2e18) ? INT64_MIN : v < 9.2e18 ? (long long)v : INT64_MAX;
+        };
+        f.yTop = state(plan.fxTop);
+        f.yBand = state(plan.fxBand);
+        const double w = plan.fxTop - plan.fxBand, top = plan.base.barSmooth / plan.base.twoSmooth;
+        if (w >= 0.0 && w < std::ldexp(0.99, -FX_SMOOTH_BITS)) f.bandScale = top * std::ldexp(1.0, -3 - 62);
+    }
+    plan.fxState = ok ? 1 : -1;
+    plan.fxIn = FxInput();
+    return ok;
+}
+
+// Range of a risk launch's vol adjoints: a slab word of 96 bits takes at most `block` paths x (steps that
+// share its time column) of them, each below 2^53 units of 2^-(60 - nodeShift).
+int fx_node_shift(const Plan& plan, int block)
+{
+    int s = 30;
+    while (s > 0 && std::ldexp(1.0, 95 - 53 - s) <= double(block) * std::max(1, plan.fxTouch)) --s;
+    return s;
+}
+
+}  // namespace cf

@@ -7,6 +7,8 @@
 #include <string>
 #include <vector>
 
+#include "fixed64.h"
+
 namespace cf {
 
 constexpr double kEps = 1.0e-08;                  // gaussians.h:8
@@ -47,6 +49,13 @@ double inv_normal_bsm(double p);
 constexpr int INVN_SUB_BITS = 4;
 constexpr int INVN_PIECES = 32 << INVN_SUB_BITS;
 void inv_normal_table(double denom, float* out /* [INVN_PIECES][4] */);
+
+// Fixed-point inverse normal (fixed64.h): the pieces of a generator and its first draw of the central
+// formula (0 when a coefficient does not fit, which no generator below does).  mrg32k3a's two
+// halves are the same function of the distance from their end; the truncated constant of the Sobol
+// uniforms makes the upper half 1 - c (2^32 - up), not c up.
+enum FxgGenerator : int { FXG_MRG = 0, FXG_SOBOL_LOWER = 1, FXG_SOBOL_UPPER = 2 };
+unsigned inv_normal_table64(int generator, FxgPiece* pieces /* [FXG_PIECES] */);
 
 // Equal buckets over the log-spot knots of the FP32 Dupire kernels: bucket b is
 // [x0 + b / invW, x0 + (b + 1) / invW) and first[b] the index of the first knot above its left

@@ -16,9 +16,15 @@ const void* mc_kernel_ptr_dupire_f32(int prod, int rng, int risk);
 const void* dupire_risk32_ptr_l1(int prod, int rng);
 const void* dupire_risk32_ptr_tma(int prod, int rng);
 size_t dupire_risk32_smem(int rng, const McParams& p);
+const void* dupire_fx64_ptr_european(int rng, int risk, int block);
+const void* dupire_fx64_ptr_uoc(int rng, int risk, int block);
+size_t dupire_fx64_smem(int rng, int block, const McParams& p);
 
 static const void* kernel_ptr(const McLaunch& l)
 {
+    if (l.fast == 3)
+        return l.prod == PROD_UOC ? dupire_fx64_ptr_uoc(l.rng, l.risk, l.block)
+                                  : dupire_fx64_ptr_european(l.rng, l.risk, l.block);
     if (l.fast) return l.fast == 2 ? dupire_risk32_ptr_tma(l.prod, l.rng) : dupire_risk32_ptr_l1(l.prod, l.rng);
     if (l.model == MODEL_BS)
         return l.fp32 ? mc_kernel_ptr_bs_f32(l.prod, l.rng, l.risk) : mc_kernel_ptr_bs_f64(l.prod, l.rng, l.risk);
@@ -28,6 +34,11 @@ static const void* kernel_ptr(const McLaunch& l)
 
 int mc_smem_bytes(const McLaunch& l, const McParams& p, int stageY, size_t* bytes)
 {
+    if (l.fast == 3)
+    {
+        *bytes = dupire_fx64_smem(l.rng, l.block, p);
+        return 0;
+    }
     *bytes = l.fast ? dupire_risk32_smem(l.rng, p) : mc_layout(l.model, l.rng, l.fp32, stageY, p, MC_BLOCK).total;
     return 0;
 }
@@ -49,16 +60,18 @@ int mc_scratch_fields(const McLaunch& l, long long rounds)
     const int NP = l.rng == RNG_SOBOL ? 1 : 2;
     // dupire_risk32, per ring slot: Gaussian, packed step word per path, and for the barrier
     // the survival factor and spot of band dates per path; generic kernel: Gaussian, state per
-    // path, and for the barrier the survival factor of band dates per path
+    // path, and for the barrier the survival factor of band dates per path (dupire_fx64: the same
+    // fields in a ring)
     const int slots = int(rounds < 1 ? 1 : rounds < R32_RING ? rounds : R32_RING);
+    if (l.fast == 3) return slots * (1 + NP + (l.prod == PROD_UOC ? NP : 0));
     if (l.fast) return slots * (1 + NP + (l.prod == PROD_UOC ? 2 * NP : 0));
     return 1 + NP + (l.prod == PROD_UOC ? NP : 0);
 }
 
 size_t mc_scratch_bytes(const McLaunch& l, McParams& p, long long grid)
 {
-    const size_t fields = size_t(p.scratchFields) * size_t(p.nSteps + 1) * size_t(grid) * 128 * (l.fp32 ? 4 : 8);
-    if (!l.fast)
+    const size_t fields = size_t(p.scratchFields) * size_t(p.nSteps + 1) * size_t(grid) * (l.fast == 3 ? l.block : MC_BLOCK) * (l.fp32 ? 4 : 8);
+    if (!l.fast || l.fast == 3)
     {
         p.nodeSlabOffset = 0;
         return fields;
@@ -128,7 +141,8 @@ int mc_occupancy(const McLaunch& l, size_t smem, int* blocksPerSM)
     if (!fn) return (int)cudaErrorInvalidDeviceFunction;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, fn, MC_BLOCK, smem);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, fn, l.fast == 3 ? l.block : MC_BLOCK,
+                                                              smem);
 }
 
 int launch_mc(const McLaunch& l, const McParams& p, void* stream)
@@ -137,7 +151,7 @@ int launch_mc(const McLaunch& l, const McParams& p, void* stream)
     if (!fn) return (int)cudaErrorInvalidDeviceFunction;
     McParams q = p;
     void* args[] = {&q};
-    return (int)cudaLaunchKernel(fn, dim3(l.grid), dim3(MC_BLOCK), args, l.smem, (cudaStream_t)stream);
+    return (int)cudaLaunchKernel(fn, dim3(l.grid), dim3(l.fast == 3 ? l.block : MC_BLOCK), args, l.smem, (cudaStream_t)stream);
 }
 
 }  // namespace cf

@@ -34,6 +34,7 @@ extern thread_local std::string g_lastError;
 
 struct Request
 {
+    bool generic = false;  // FP64 risk in double arithmetic (smaller scratch)
     int kind = 0;  // 0 value, 1 risk (weights), 2 multi
     std::string mid, pid;
     cf_num_param num{};
@@ -104,7 +105,7 @@ public:
                 if (j.lane == 1 && chunkPathSteps > 0)
                     chunk = std::max(64LL, (long long)(chunkPathSteps / std::max(1, plan->nSteps)) & ~63LL);
                 rc = c.enqueue(*slots[s], *plan, r.num, r.kind == 1, r.w.empty() ? nullptr : r.w.data(), 0, nullptr,
-                               chunk, j.lane == 1 ? longBlocksPerSM : 0);
+                               chunk, j.lane == 1 ? longBlocksPerSM : 0, r.generic);
             }
         }
         if (rc) err = g_lastError;
@@ -294,7 +295,14 @@ int cf_server_submit(cf_server* s, const cf_request* r, uint64_t* id)
     q.pid = r->productId;
     q.num = r->num;
     if (r->weights) q.w.assign(r->weights, r->weights + r->nWeights);
-    const size_t fp = s->ctx->c.footprint(*plan, r->num, r->kind != 0);
+    size_t fp = s->ctx->c.footprint(*plan, r->num, r->kind != 0);
+    if (fp > s->sched.budget() && r->kind == 1)
+    {
+        // an FP64 risk whose ring of round slots exceeds the budget runs the generic kernel
+        const size_t small = s->ctx->c.footprint(*plan, r->num, true, true);
+        q.generic = small < fp;
+        fp = std::min(fp, small);
+    }
     const long long work = (long long)r->num.numPath * plan->nSteps;
     {
         std::lock_guard<std::mutex> b(s->mu);

@@ -74,6 +74,7 @@ public:
     }
     int laneOrder(int lane) const { return lane < int(order_.size()) ? order_[lane] : 0; }
 
+    size_t budget() const { return budget_; }
     // Registers a request; a request larger than the whole budget is rejected at once.
     uint64_t submit(size_t footprint, double queueTimeout, double now, long long work = 0, int lane = 0)
     {

@@ -76,8 +76,7 @@ int bump_risk_pathwise(Context& c, Plan& plan, const ModelDesc& m, const Product
     p.nPath = num.numPath;
     p.seed1 = unsigned(num.seed1);
     p.seed2 = unsigned(num.seed2);
-    p.mrgJumpA = c.jumpA;
-    p.mrgJumpB = c.jumpB;
+    c.setGenerator(p, sobol);
     BumpArgs b{};
     b.nParam = nParam;
     b.maskWords = (p.nS * p.nT + 31) / 32;

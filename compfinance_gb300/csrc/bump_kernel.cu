@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(BB) dupire_bump64(const McParams p, const Bump
         MrgState st = mrg_jump(p.seed1, p.seed2, (unsigned long long)u0 * nSteps, p.mrgJumpA, p.mrgJumpB);
         for (long long u = u0; u < u1; ++u)
         {
-            for (int s = 0; s < nSteps; ++s) D(R.dG + s) = mrg_gauss<double>(mrg_next(st));
+            for (int s = 0; s < nSteps; ++s) D(R.dG + s) = mrg_gauss<double>(p.fx, mrg_next(st));
             runPath(0);
             if (2 * u + 1 < p.nPath) runPath(1);
         }
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(BB) dupire_bump64(const McParams p, const Bump
         // Sobol: index n = 1 .. nPath (path n - 1), strided over the grid
         for (long long n = tg + 1; n <= p.nPath; n += Ti)
         {
-            for (int s = 0; s < nSteps; ++s) D(R.dG + s) = sobol_gauss<double>(sobol_state(p.sobolDir, nSteps, s, n));
+            for (int s = 0; s < nSteps; ++s) D(R.dG + s) = sobol_gauss<double>(p.fx, sobol_state(p.sobolDir, nSteps, s, n));
             runPath(0);
         }
     }

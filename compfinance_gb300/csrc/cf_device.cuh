@@ -304,18 +304,50 @@ __device__ __forceinline__ float sobol_gauss_f(unsigned s)
     return inv_normal_up(__int2float_rn(int(up - (up >> 31))) * 2.3283064365386963e-10f, sup);
 }
 
+// Fixed-point Gaussian (fixed64.h) in units of 2^-59 of a draw at distance up from the end of its
+// half (sup: the upper one).
+template <bool SOBOL>
+__device__ __forceinline__ long long fx_gauss(const FxParams& f, unsigned up, bool sup)
+{
+    const bool upper = SOBOL && sup;
+    int w;
+    const int k = fxg_piece(up, upper ? f.brk[1] : f.brk[0], w);
+    const longlong2* c = reinterpret_cast<const longlong2*>((upper ? f.g[1] : f.g[0]) + k);
+    const longlong2 c0 = __ldg(c), c1 = __ldg(c + 1);
+    const long long g = fxg_value(FxgPiece{c0.x, c0.y, c1.x, (int)c1.y, (int)(c1.y >> 32)}, w);
+    return sup ? g : -g;
+}
+__device__ __forceinline__ long long mrg_gauss_fx(const FxParams& f, unsigned d)
+{
+    const bool sup = d > 2147483544u;  // (m1 + 1) / 2
+    return fx_gauss<false>(f, sup ? 4294967088u - d : d, sup);
+}
+__device__ __forceinline__ long long sobol_gauss_fx(const FxParams& f, unsigned s)
+{
+    const bool sup = s >= 2147483648u;
+    return fx_gauss<true>(f, sup ? 0u - s : (s > 1u ? s : 1u), sup);  // state 0 occurs only at index 0
+}
+
+// Gaussians of the path kernels.  In doubles, the table's value converted: two FP64 operations where
+// the formula takes about 105 (a warp's lanes nearly always need both of its branches).
 template <class Real>
-__device__ __forceinline__ Real mrg_gauss(unsigned d);
+__device__ __forceinline__ Real mrg_gauss(const FxParams& f, unsigned d);
 template <>
-__device__ __forceinline__ double mrg_gauss<double>(unsigned d) { return mrg_gauss_d(d); }
+__device__ __forceinline__ double mrg_gauss<double>(const FxParams& f, unsigned d)
+{
+    return (double)mrg_gauss_fx(f, d) * 0x1p-59;
+}
 template <>
-__device__ __forceinline__ float mrg_gauss<float>(unsigned d) { return mrg_gauss_f(d); }
+__device__ __forceinline__ float mrg_gauss<float>(const FxParams&, unsigned d) { return mrg_gauss_f(d); }
 template <class Real>
-__device__ __forceinline__ Real sobol_gauss(unsigned s);
+__device__ __forceinline__ Real sobol_gauss(const FxParams& f, unsigned s);
 template <>
-__device__ __forceinline__ double sobol_gauss<double>(unsigned s) { return sobol_gauss_d(s); }
+__device__ __forceinline__ double sobol_gauss<double>(const FxParams& f, unsigned s)
+{
+    return (double)sobol_gauss_fx(f, s) * 0x1p-59;
+}
 template <>
-__device__ __forceinline__ float sobol_gauss<float>(unsigned s) { return sobol_gauss_f(s); }
+__device__ __forceinline__ float sobol_gauss<float>(const FxParams&, unsigned s) { return sobol_gauss_f(s); }
 
 // Sobol point of index n (path n-1): XOR of direction numbers over the set bits of gray(n)
 // (sobol.h:119-151).  dir is [32][stride] for the dimensions of the launch.

@@ -761,6 +761,7 @@ int Context::init(int dev)
     CF_CUDA(cudaMemcpy(invn.ptr, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
     invnMrg = static_cast<const float*>(invn.ptr);
     invnSobol = invnMrg + size_t(INVN_PIECES) * 4;
+    if ((rc = initGauss())) return rc;
     main.stream = stream;
     return CF_OK;
 }
@@ -824,9 +825,7 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     p.firstPath = firstPath;
     p.seed1 = unsigned(num.seed1);
     p.seed2 = unsigned(num.seed2);
-    p.mrgJumpA = jumpA;
-    p.mrgJumpB = jumpB;
-    p.invnF = sobol ? invnSobol : invnMrg;
+    setGenerator(p, sobol);
     p.nRisk = risk ? plan.nParam : 0;
     p.nAcc = p.nRisk + 2 * plan.nPay + 2;
     p.pathOut = risk ? nullptr : pathOut;
@@ -871,14 +870,10 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     // FP64 Dupire European and barrier runs in fixed point at every size their tables fit: 60x30 weekly
     // barrier risk 9.5 -> 0.62 ms at 2^18 paths (141 -> 5.6 ms at 2^22), its value 5.2 -> 0.30 ms,
     // 20x10 grid and 10^5 x 52 steps 0.85 -> 0.14 ms against the generic kernel
-    if (!fp32 && !generic && fxReady(plan) && fxGauss(sobol))
+    if (!fp32 && !generic && fxReady(plan))
     {
         p.fx = plan.fx;
-        const int g0 = sobol ? FXG_SOBOL_LOWER : FXG_MRG, g1 = sobol ? FXG_SOBOL_UPPER : FXG_MRG;
-        p.fx.g[0] = static_cast<const FxgPiece*>(fxg[sobol ? 1 : 0].ptr);
-        p.fx.g[1] = p.fx.g[0] + (sobol ? FXG_PIECES : 0);
-        p.fx.brk[0] = fxgBrk[g0];
-        p.fx.brk[1] = fxgBrk[g1];
+        setGenerator(p, sobol);
         l.fast = 3;
         // a node slab of many nodes is shared by a larger block when that keeps more threads resident
         int best = 0, block = 128;

@@ -187,7 +187,7 @@ struct Context
     DevBuf invn;  // piecewise-cubic inverse normal tables of the FP32 kernels: mrg32k3a, Sobol
     const float* invnMrg = nullptr;
     const float* invnSobol = nullptr;
-    DevBuf fxg[2];  // fixed-point inverse normal of mrg32k3a and of Sobol's two halves (fx_plan.cpp)
+    DevBuf fxg;  // fixed-point inverse normal of mrg32k3a and of Sobol's two halves (fixed64.h)
     unsigned fxgBrk[3] = {0, 0, 0};
     Slot main;
     unsigned long long h2d = 0, d2h = 0;  // cumulative transfer bytes
@@ -211,9 +211,11 @@ struct Context
     int enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk, const double* weights,
                 long long firstPath = 0, double* pathOut = nullptr, long long chunkPaths = 0,
                 int maxBlocksPerSM = 0, bool generic = false);
-    // fx_plan.cpp: the fixed-point tables of a plan and of a generator, built on first use
+    // fx_plan.cpp: the tables of the inverse normal, a launch's generator parameters (jump tables and
+    // inverse normals), and the fixed-point tables of a plan, built on first use
+    int initGauss();
+    void setGenerator(McParams& p, bool sobol) const;
     bool fxReady(Plan& plan);
-    bool fxGauss(bool sobol);
     int fetch(Slot& slot, double* values, double* stderrs, double* aggregate, double* risks);
     bool ready(Slot& slot) const;
     size_t footprint(const Plan& plan, const cf_num_param& num, bool risk, bool generic = false) const;

@@ -10,21 +10,38 @@
 
 namespace cf {
 
-// The inverse normal's pieces of a generator (20 ms of host work per table), on first use; Sobol's two
-// halves have a table each.
-bool Context::fxGauss(bool sobol)
+// The generators' inverse normal tables, made once per process (20 ms of host work each).
+static const std::vector<FxgPiece>& gauss_tables(unsigned brk[3])
 {
-    DevBuf& buf = fxg[sobol ? 1 : 0];
-    if (buf.ptr) return true;
-    const int first = sobol ? FXG_SOBOL_LOWER : FXG_MRG, n = sobol ? 2 : 1;
-    std::vector<FxgPiece> g(size_t(n) * FXG_PIECES);
-    bool ok = true;
-    for (int k = 0; k < n; ++k)
-        ok = (fxgBrk[first + k] = inv_normal_table64(first + k, &g[size_t(k) * FXG_PIECES])) != 0 && ok;
-    const size_t bytes = g.size() * sizeof(FxgPiece);
-    ok = ok && buf.ensure(bytes) == CF_OK && cudaMemcpy(buf.ptr, g.data(), bytes, cudaMemcpyHostToDevice) == cudaSuccess;
-    if (!ok) buf.release();
-    return ok;
+    static unsigned breaks[3];
+    static const std::vector<FxgPiece> tables = [] {
+        std::vector<FxgPiece> g(size_t(3) * FXG_PIECES);
+        for (int k = 0; k < 3; ++k) breaks[k] = inv_normal_table64(k, &g[size_t(k) * FXG_PIECES]);
+        return g;
+    }();
+    std::copy(breaks, breaks + 3, brk);
+    return tables;
+}
+
+int Context::initGauss()
+{
+    const std::vector<FxgPiece>& g = gauss_tables(fxgBrk);
+    int rc = fxg.ensure(g.size() * sizeof(FxgPiece));
+    if (rc) return rc;
+    CF_CUDA(cudaMemcpy(fxg.ptr, g.data(), g.size() * sizeof(FxgPiece), cudaMemcpyHostToDevice));
+    return CF_OK;
+}
+
+void Context::setGenerator(McParams& p, bool sobol) const
+{
+    p.mrgJumpA = jumpA;
+    p.mrgJumpB = jumpB;
+    p.invnF = sobol ? invnSobol : invnMrg;
+    const FxgPiece* g = static_cast<const FxgPiece*>(fxg.ptr);
+    p.fx.g[0] = g + size_t(sobol ? FXG_SOBOL_LOWER : FXG_MRG) * FXG_PIECES;
+    p.fx.g[1] = g + size_t(sobol ? FXG_SOBOL_UPPER : FXG_MRG) * FXG_PIECES;
+    p.fx.brk[0] = fxgBrk[sobol ? FXG_SOBOL_LOWER : FXG_MRG];
+    p.fx.brk[1] = fxgBrk[sobol ? FXG_SOBOL_UPPER : FXG_MRG];
 }
 
 bool Context::fxReady(Plan& plan)

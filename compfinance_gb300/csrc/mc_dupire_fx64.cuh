@@ -117,17 +117,6 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
         const int4 c = __ldg(reinterpret_cast<const int4*>(vols + s * pitch + lo));
         return fx_vol((long long)(((unsigned long long)(unsigned)c.y << 32) | (unsigned)c.x), c.z, c.w, y, center, dShift);
     };
-    // Gaussian of a draw at distance up from the end of its half, in units of 2^-59
-    auto gauss = [&](unsigned up, bool sup) -> long long {
-        const bool upper = RNGK == RNG_SOBOL && sup;
-        int w;
-        const int k = fxg_piece(up, upper ? p.fx.brk[1] : p.fx.brk[0], w);
-        const longlong2* c = reinterpret_cast<const longlong2*>((upper ? p.fx.g[1] : p.fx.g[0]) + k);
-        const longlong2 c0 = __ldg(c), c1 = __ldg(c + 1);
-        const long long g = fxg_value(FxgPiece{c0.x, c0.y, c1.x, (int)c1.y, (int)(c1.y >> 32)}, w);
-        return sup ? g : -g;
-    };
-
     // scratch [ring slot][field][point][thread] of 64-bit words, 32-bit offsets: the Gaussian, the
     // state per path and, for the barrier, the survival factor before band dates per path.  Point
     // nSteps holds the adjoint seeds of the state and of the survival factor.
@@ -442,11 +431,7 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
                 const long long u = u0 + j;
                 const int nAct = u < nUnits ? ((2 * u + 1 < p.nPath) ? 2 : 1) : 0;
                 const int slot = RISK ? slotOf(it) : 0;
-                forward(nAct, 2 * u, [&](int) {
-                    const unsigned d = mrg_next(st);   // in [1, m1]; uniform d / (m1 + 1)
-                    const bool sup = d > 2147483544u;  // (m1 + 1) / 2
-                    return gauss(sup ? 4294967088u - d : d, sup);
-                });
+                forward(nAct, 2 * u, [&](int) { return mrg_gauss_fx(p.fx, mrg_next(st)); });
                 if (RISK) endRound(slot);
             }
         }
@@ -476,9 +461,7 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
                 }
                 const int slot = RISK ? slotOf(it) : 0;
                 forward(nAct, n - 1, [&](int i) {
-                    const unsigned sb = base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane);
-                    const bool sup = sb >= 2147483648u;
-                    return gauss(sup ? 0u - sb : (sb > 1u ? sb : 1u), sup);  // state 0 occurs only at index 0
+                    return sobol_gauss_fx(p.fx, base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
                 });
                 if (RISK) endRound(slot);
             }

@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
             {
                 const long long u = u0 + j;
                 const int nAct = u < nUnits ? ((2 * u + 1 < p.nPath) ? 2 : 1) : 0;
-                if (ROWACC || nAct) runUnit(nAct, 2 * u, [&](int) { return mrg_gauss<Real>(mrg_next(st)); });
+                if (ROWACC || nAct) runUnit(nAct, 2 * u, [&](int) { return mrg_gauss<Real>(p.fx, mrg_next(st)); });
                 if (ROWACC && (it + 1) % p.nodeFlushUnits == 0) flushNodes();
             }
         }
@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
                 const int nAct = (n >= 1 && n <= p.nPath) ? 1 : 0;
                 if (ROWACC || nAct)
                     runUnit(nAct, n - 1, [&](int i) {
-                        return sobol_gauss<Real>(base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
+                        return sobol_gauss<Real>(p.fx, base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
                     });
             }
         }

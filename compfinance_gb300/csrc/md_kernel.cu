@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
             MrgState st = mrg_jump(p.seed1, p.seed2, (unsigned long long)(p.firstPath / 2 + u0) * dim, p.mrgJumpA,
                                    p.mrgJumpB);
             for (long long u = u0; u < u1; ++u)
-                runUnit((2 * u + 1 < p.nPath) ? 2 : 1, [&](int) { return mrg_gauss<Real>(mrg_next(st)); });
+                runUnit((2 * u + 1 < p.nPath) ? 2 : 1, [&](int) { return mrg_gauss<Real>(p.fx, mrg_next(st)); });
         }
     }
     else
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
             const long long n = b * 32 + lane;
             if (n >= 1 && n <= p.nPath)
                 runUnit(1, [&](int d) {
-                    return sobol_gauss<Real>(base[d] ^ sobol_state(p.sobolDir, dim, d, (unsigned long long)lane));
+                    return sobol_gauss<Real>(p.fx, base[d] ^ sobol_state(p.sobolDir, dim, d, (unsigned long long)lane));
                 });
         }
     }

@@ -136,8 +136,7 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
     p.nPath = num.numPath;
     p.seed1 = unsigned(num.seed1);
     p.seed2 = unsigned(num.seed2);
-    p.mrgJumpA = jumpA;
-    p.mrgJumpB = jumpB;
+    setGenerator(p, sobol);
     p.err = reinterpret_cast<int*>(d + offErr);
     p.claim = reinterpret_cast<unsigned long long*>(d + offErr + 64);  // multi32_forward's Sobol batch counter
     const int* dEvOff = reinterpret_cast<const int*>(d);
@@ -148,7 +147,6 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
         // FP32 Dupire: forward, bucket segments, chunked reverse sweeps (multi_risk32.cu)
         Multi32Args A;
         A.p = p;
-        A.p.invnF = sobol ? invnSobol : invnMrg;
         A.nParam = nParam;
         A.nBuckets = nBuckets;
         A.nKs = int(ksf.size());

@@ -316,8 +316,7 @@ int Context::enqueueMd(Slot& slot, Plan& plan, const cf_num_param& num, bool ris
     p.firstPath = firstPath;
     p.seed1 = unsigned(num.seed1);
     p.seed2 = unsigned(num.seed2);
-    p.mrgJumpA = jumpA;
-    p.mrgJumpB = jumpB;
+    setGenerator(p, sobol);
     p.nRisk = risk ? plan.mdTotal : 0;
     p.nAcc = p.nRisk + 2 * plan.nPay + 2;
     const size_t wBytes = ((size_t(plan.nPay) * 12 + 255) & ~size_t(255));

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(MC_BLOCK) multi_kernel(const MultiParams mp)
         {
             MrgState st = mrg_jump(p.seed1, p.seed2, (unsigned long long)(p.firstPath / 2 + u0) * nSteps, p.mrgJumpA, p.mrgJumpB);
             for (long long u = u0; u < u1; ++u)
-                runUnit((2 * u + 1 < p.nPath) ? 2 : 1, [&](int) { return mrg_gauss<Real>(mrg_next(st)); });
+                runUnit((2 * u + 1 < p.nPath) ? 2 : 1, [&](int) { return mrg_gauss<Real>(p.fx, mrg_next(st)); });
         }
     }
     else
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(MC_BLOCK) multi_kernel(const MultiParams mp)
             const long long n = b * 32 + lane;
             if (n >= 1 && n <= p.nPath)
                 runUnit(1, [&](int i) {
-                    return sobol_gauss<Real>(base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
+                    return sobol_gauss<Real>(p.fx, base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
                 });
         }
     }

@@ -328,6 +328,16 @@ __device__ __forceinline__ long long sobol_gauss_fx(const FxParams& f, unsigned 
     return fx_gauss<true>(f, sup ? 0u - s : (s > 1u ? s : 1u), sup);  // state 0 occurs only at index 0
 }
 
+// exp(x) of the FP64 kernels: integer work and three FP64 operations, where exp() takes 20.
+__device__ __forceinline__ double exp_fx(const FxParams& f, double x)
+{
+    if ((unsigned(__double2hiint(x)) & 0x7fffffffu) >= 0x402f0000u) return exp(x);  // |x| >= 15.5, NaN
+    int n;
+    const double m = (double)fx_exp(f.expTab, __double2ll_rn(x * 0x1p58), n);
+    return __hiloint2double(__double2hiint(m) + ((n - 61) << 20), __double2loint(m));
+}
+__device__ __forceinline__ float exp_fx(const FxParams&, float x) { return exp(x); }
+
 // Gaussians of the path kernels.  In doubles, the table's value converted: two FP64 operations where
 // the formula takes about 105 (a warp's lanes nearly always need both of its branches).
 template <class Real>

@@ -97,6 +97,7 @@ struct FxParams
     // spot; bandScale > 0: the factor is bandScale times fx_one_minus_exp8(yTop - y)
     long long yTop, yBand;
     double bandScale;
+    const long long* expTab;     // table of fx_exp
     // inverse normal: pieces of the generator's lower and upper halves
     const FxgPiece* g[2];
     unsigned brk[2];

@@ -187,7 +187,7 @@ struct Context
     DevBuf invn;  // piecewise-cubic inverse normal tables of the FP32 kernels: mrg32k3a, Sobol
     const float* invnMrg = nullptr;
     const float* invnSobol = nullptr;
-    DevBuf fxg;  // fixed-point inverse normal of mrg32k3a and of Sobol's two halves (fixed64.h)
+    DevBuf fxg;  // tables of fixed64.h: inverse normal of mrg32k3a and of Sobol's two halves, exponential
     unsigned fxgBrk[3] = {0, 0, 0};
     Slot main;
     unsigned long long h2d = 0, d2h = 0;  // cumulative transfer bytes

@@ -10,25 +10,31 @@
 
 namespace cf {
 
-// The generators' inverse normal tables, made once per process (20 ms of host work each).
-static const std::vector<FxgPiece>& gauss_tables(unsigned brk[3])
+// The generators' inverse normal tables and the exponential's, made once per process (20 ms of host
+// work for each of the former).
+namespace {
+struct Tables
 {
-    static unsigned breaks[3];
-    static const std::vector<FxgPiece> tables = [] {
-        std::vector<FxgPiece> g(size_t(3) * FXG_PIECES);
-        for (int k = 0; k < 3; ++k) breaks[k] = inv_normal_table64(k, &g[size_t(k) * FXG_PIECES]);
-        return g;
-    }();
-    std::copy(breaks, breaks + 3, brk);
-    return tables;
-}
+    std::vector<FxgPiece> g;
+    unsigned brk[3];
+    long long e[1 << FX_EXP_BITS];
+    Tables() : g(size_t(3) * FXG_PIECES)
+    {
+        for (int k = 0; k < 3; ++k) brk[k] = inv_normal_table64(k, &g[size_t(k) * FXG_PIECES]);
+        exp_table64(e);
+    }
+};
+}  // namespace
 
 int Context::initGauss()
 {
-    const std::vector<FxgPiece>& g = gauss_tables(fxgBrk);
-    int rc = fxg.ensure(g.size() * sizeof(FxgPiece));
+    static const Tables t;
+    std::copy(t.brk, t.brk + 3, fxgBrk);
+    const size_t n = t.g.size() * sizeof(FxgPiece);
+    int rc = fxg.ensure(n + sizeof(t.e));
     if (rc) return rc;
-    CF_CUDA(cudaMemcpy(fxg.ptr, g.data(), g.size() * sizeof(FxgPiece), cudaMemcpyHostToDevice));
+    CF_CUDA(cudaMemcpy(fxg.ptr, t.g.data(), n, cudaMemcpyHostToDevice));
+    CF_CUDA(cudaMemcpy(static_cast<char*>(fxg.ptr) + n, t.e, sizeof(t.e), cudaMemcpyHostToDevice));
     return CF_OK;
 }
 
@@ -40,6 +46,7 @@ void Context::setGenerator(McParams& p, bool sobol) const
     const FxgPiece* g = static_cast<const FxgPiece*>(fxg.ptr);
     p.fx.g[0] = g + size_t(sobol ? FXG_SOBOL_LOWER : FXG_MRG) * FXG_PIECES;
     p.fx.g[1] = g + size_t(sobol ? FXG_SOBOL_UPPER : FXG_MRG) * FXG_PIECES;
+    p.fx.expTab = reinterpret_cast<const long long*>(g + size_t(3) * FXG_PIECES);
     p.fx.brk[0] = fxgBrk[sobol ? FXG_SOBOL_LOWER : FXG_MRG];
     p.fx.brk[1] = fxgBrk[sobol ? FXG_SOBOL_UPPER : FXG_MRG];
 }

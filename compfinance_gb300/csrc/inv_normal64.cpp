@@ -1,4 +1,4 @@
-// Tables of the fixed-point inverse normal (fixed64.h): Beasley-Springer-Moro (gaussians.h:47-87)
+// Tables of the fixed-point exponential and inverse normal (fixed64.h), the latter Beasley-Springer-Moro (gaussians.h:47-87)
 // evaluated in double-double arithmetic at five Chebyshev nodes of every piece.  The tables are
 // built once per context.  Compiled with -ffp-contract=off.
 #include <algorithm>
@@ -103,6 +103,20 @@ long long to_fixed(const DD& v, int shift)
 }
 
 }  // namespace
+
+void exp_table64(long long* out)
+{
+    // 2^(1/128) by seven square roots of 2 (Newton steps of r - (r^2 - a) / (2 r)), then its powers
+    DD root(2.0);
+    for (int k = 0; k < FX_EXP_BITS; ++k)
+    {
+        DD r(std::sqrt(root.hi));
+        for (int i = 0; i < 2; ++i) r = r - (r * r - root) / (r + r);
+        root = r;
+    }
+    DD p(1.0);
+    for (int i = 0; i < (1 << FX_EXP_BITS); ++i, p = p * root) out[i] = to_fixed(p, 61);
+}
 
 unsigned inv_normal_table64(int gen, FxgPiece* out)
 {

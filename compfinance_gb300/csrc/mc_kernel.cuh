@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
                 }
                 else
                 {
-                    x[a] = x[a] * exp(bs[i] + bs[nSteps + i] * ga);
+                    x[a] = x[a] * exp_fx(p.fx, bs[i] + bs[nSteps + i] * ga);
                 }
             }
             const int e = p.evAtStep[i + 1];
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
                 }
                 else
                 {
-                    const Real E = exp(bs[s] + bs[nSteps + s] * ga);
+                    const Real E = exp_fx(p.fx, bs[s] + bs[nSteps + s] * ga);
                     const Real aArg = ax[a] * (xs * E);  // d S_{s+1} / d(drift + std g) = S_{s+1}
                     aVol[a] += aArg * bs[4 * nSteps + s] + aArg * ga * bs[3 * nSteps + s];
                     aR[a] += aArg * bs[2 * nSteps + s];

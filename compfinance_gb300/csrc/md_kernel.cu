@@ -39,7 +39,7 @@ __device__ __forceinline__ const float* pickR<float>(const double*, const float*
 
 struct MdSmem
 {
-    size_t acc, tab, asset, strike, weight, dyn, base, total;
+    size_t acc, tab, asset, strike, weight, inv, dyn, base, total;
 };
 
 // shared memory: accumulators, derived table, per-asset and per-payoff constants, Sobol bases
@@ -59,6 +59,7 @@ __host__ __device__ inline MdSmem md_smem(int rng, int fp32, const McParams& p)
     S.asset = take(size_t(p.nA) * rs);
     S.strike = take(size_t(p.nPay) * rs);
     S.weight = take(size_t(p.nPay) * rs);
+    S.inv = take(fp32 ? 0 : size_t(p.nA + p.nEv) * 8);  // reciprocals of the references and the numeraires
     S.dyn = take(size_t(p.nA) * 4);
     S.base = take(rng == RNG_SOBOL ? size_t(MD_BLOCK / 32) * (size_t(p.nSteps * p.nA) | 1) * 4 : 0);
     S.total = off;
@@ -83,9 +84,11 @@ __device__ __forceinline__ void md_add(long long* slot, double v)
     }
 }
 
-// FP64, up to four assets: five blocks per SM (four with mrg32k3a, which carries two paths)
+// Resident blocks per SM asked for up to four assets (mrg32k3a carries two paths): FP64 5 and 4
+// (96 and 128 registers), FP32 8 and 6 (64 and 80).
 template <int RNGK, class Real, int NA>
-__global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RNGK == RNG_SOBOL ? 5 : 4) md_kernel(const McParams p)
+__global__ void __launch_bounds__(MD_BLOCK, NA > 4 ? 1 : sizeof(Real) == 4 ? (RNGK == RNG_SOBOL ? 8 : 6) : RNGK == RNG_SOBOL ? 5 : 4)
+    md_kernel(const McParams p)
 {
     constexpr int NP = RNGK == RNG_MRG ? 2 : 1;
     constexpr bool F32 = std::is_same<Real, float>::value;
@@ -96,6 +99,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
     Real* sAsset = reinterpret_cast<Real*>(smem + S.asset);
     Real* sK = reinterpret_cast<Real*>(smem + S.strike);
     Real* sW = reinterpret_cast<Real*>(smem + S.weight);
+    Real* sInv = reinterpret_cast<Real*>(smem + S.inv);
     int* sDyn = reinterpret_cast<int*>(smem + S.dyn);
     const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
     const int nA = p.nA, nSteps = p.nSteps, nEv = p.nEv, nPay = p.nPay, nRisk = p.nRisk, dim = nSteps * nA;
@@ -113,7 +117,10 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
         {
             sAsset[i] = gAsset[i];
             sDyn[i] = p.mdDyn[i];
+            if (!F32) sInv[i] = Real(1) / gAsset[i];
         }
+        if (!F32)
+            for (int i = tid; i < nEv; i += MD_BLOCK) sInv[nA + i] = Real(1) / gTab[L.num + i];
         for (int i = tid; i < nPay; i += MD_BLOCK)
         {
             sK[i] = basket ? gK[i] : Real(0);
@@ -126,6 +133,8 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
     const Real ko = Real(p.acKo), kput = Real(p.acStrike), cpn = Real(p.acCpn), dtc = Real(p.acDt),
                sm = Real(p.acSmooth);
 
+    const Real halfInv = Real(0.5) / sm, putInv = Real(1) / kput;
+
     // reverse-sweep scratch [field][thread]: Gaussians [dim], spots after each step [NP][dim],
     // autocall notional alive before each date [NP][nEv]
     const long long T = (long long)gridDim.x * MD_BLOCK;
@@ -136,7 +145,29 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
     auto SA = [&](int a, int e) -> Real& { return scr[size_t(dim + NP * dim + a * nEv + e) * T]; };
 
     // worst performance at date e (the first minimum, as min_element), its asset
+    // FP64 form: a division takes ten times a product there, so the first minimum is found from products
+    // with the references' reciprocals and only its performance is divided; the divisions by a date's
+    // numeraire and by constants are products with their reciprocals
+    auto over = [](Real a, Real b, Real inv) { return F32 ? a / b : a * inv; };
     auto worstOf = [&](const Real* s, int& wi) {
+        if constexpr (!F32)
+        {
+            Real w = s[0] * sInv[0], sw = s[0];
+            wi = 0;
+#pragma unroll
+            for (int a = 1; a < NA; ++a)
+                if (a < nA)
+                {
+                    const Real q = s[a] * sInv[a];
+                    if (q < w)
+                    {
+                        w = q;
+                        sw = s[a];
+                        wi = a;
+                    }
+                }
+            return sw / sAsset[wi];
+        }
         Real w = s[0] / sAsset[0];
         wi = 0;
 #pragma unroll
@@ -190,17 +221,17 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
                     const Real c = ap ? -cw : cw;
                     const Real fwd = s[ap][a] * ff;
                     Real nx;
-                    if (dy == MD_LOGNORMAL) nx = fwd * exp(dr + sd * c);
+                    if (dy == MD_LOGNORMAL) nx = fwd * exp_fx(p.fx, dr + sd * c);
                     else if (dy == MD_NORMAL) nx = fwd + sd * c;
-                    else if (dy == MD_SURNORMAL) nx = (fwd + al) * exp(dr + sd * c) - al;
-                    else nx = (fwd - al) * exp(dr + sd * c) + al;
+                    else if (dy == MD_SURNORMAL) nx = (fwd + al) * exp_fx(p.fx, dr + sd * c) - al;
+                    else nx = (fwd - al) * exp_fx(p.fx, dr + sd * c) + al;
                     s[ap][a] = nx;
                     if (risk) SS(ap, i * nA + a) = nx;
                 }
             }
             const int e = p.evAtStep[i + 1];
             if (e < 0) continue;
-            const Real num = tab[L.num + e];
+            const Real num = tab[L.num + e], ni = F32 ? Real(0) : sInv[nA + e];
 #pragma unroll
             for (int ap = 0; ap < NP; ++ap)
             {
@@ -215,7 +246,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
                     for (int k = 0; k < nPay; ++k)
                     {
                         const Real m = b - sK[k];
-                        const Real v = (m > Real(0) ? m : Real(0)) / num;
+                        const Real v = over(m > Real(0) ? m : Real(0), num, ni);
                         md_add<NA>(&accPay[2 * k], v);
                         md_add<NA>(&accPay[2 * (nPay + k)], v * v);
                         agg += sW[k] * v;
@@ -228,20 +259,20 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
                 if (risk) SA(ap, e) = alive[ap];
                 int wi;
                 const Real worst = worstOf(s[ap], wi);
-                pay[ap] += alive[ap] * cpn * dtc / num;
+                pay[ap] += over(alive[ap] * cpn * dtc, num, ni);
                 if (e < nEv - 1)
                 {
-                    const Real x = (ko + sm - worst) / Real(2) / sm;
+                    const Real x = F32 ? (ko + sm - worst) / Real(2) / sm : (ko + sm - worst) * halfInv;
                     const Real f = x > Real(1) ? Real(1) : x > Real(0) ? x : Real(0);
                     const Real surv = alive[ap] * f;
-                    pay[ap] += (alive[ap] - surv) / num;
+                    pay[ap] += over(alive[ap] - surv, num, ni);
                     alive[ap] = surv;
                 }
                 else
                 {
-                    pay[ap] += alive[ap] / num;
+                    pay[ap] += over(alive[ap], num, ni);
                     const Real m = kput - worst;
-                    pay[ap] -= alive[ap] * (m > Real(0) ? m : Real(0)) / kput / num;
+                    pay[ap] -= over(over(alive[ap] * (m > Real(0) ? m : Real(0)), kput, putInv), num, ni);
                     md_add<NA>(&accPay[0], pay[ap]);
                     md_add<NA>(&accPay[2 * nPay], pay[ap] * pay[ap]);
                     const Real agg = sW[0] * pay[ap];
@@ -269,7 +300,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
                 const int e = p.evAtStep[i + 1];
                 if (e >= 0)
                 {
-                    const Real num = tab[L.num + e];
+                    const Real num = tab[L.num + e], ni = F32 ? Real(0) : sInv[nA + e];
                     Real sp[NA];
 #pragma unroll
                     for (int a = 0; a < NA; ++a) sp[a] = a < nA ? SS(ap, i * nA + a) : Real(0);
@@ -285,8 +316,8 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
                             const Real m = b - sK[k];
                             if (m > Real(0))
                             {
-                                bb += sW[k] / num;
-                                nb -= sW[k] * (m / num) / num;
+                                bb += over(sW[k], num, ni);
+                                nb -= over(sW[k] * over(m, num, ni), num, ni);
                             }
                         }
 #pragma unroll
@@ -304,24 +335,24 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
                         {
                             const Real m = kput - worst;
                             const Real put = m > Real(0) ? m : Real(0);
-                            payE = A * cpn * dtc / num + A / num - A * put / kput / num;
-                            aliveBar = w0 * (cpn * dtc + Real(1) - put / kput) / num;
-                            worstBar = m > Real(0) ? w0 * A / kput / num : Real(0);
+                            payE = over(A * cpn * dtc, num, ni) + over(A, num, ni) - over(over(A * put, kput, putInv), num, ni);
+                            aliveBar = over(w0 * (cpn * dtc + Real(1) - over(put, kput, putInv)), num, ni);
+                            worstBar = m > Real(0) ? over(over(w0 * A, kput, putInv), num, ni) : Real(0);
                         }
                         else
                         {
-                            const Real x = (ko + sm - worst) / Real(2) / sm;
+                            const Real x = F32 ? (ko + sm - worst) / Real(2) / sm : (ko + sm - worst) * halfInv;
                             const bool inside = x > Real(0) && x < Real(1);
                             const Real f = x > Real(1) ? Real(1) : x > Real(0) ? x : Real(0);
-                            payE = A * cpn * dtc / num + (A - A * f) / num;
-                            const Real fBar = -w0 * A / num + aliveBar * A;
-                            aliveBar = w0 * (cpn * dtc + Real(1) - f) / num + aliveBar * f;
-                            worstBar = inside ? -fBar / Real(2) / sm : Real(0);
+                            payE = over(A * cpn * dtc, num, ni) + over(A - A * f, num, ni);
+                            const Real fBar = over(-w0 * A, num, ni) + aliveBar * A;
+                            aliveBar = over(w0 * (cpn * dtc + Real(1) - f), num, ni) + aliveBar * f;
+                            worstBar = inside ? (F32 ? -fBar / Real(2) / sm : -fBar * halfInv) : Real(0);
                         }
-                        md_add<NA>(&sAcc[2 * (L.num + e)], -w0 * payE / num);
+                        md_add<NA>(&sAcc[2 * (L.num + e)], over(-w0 * payE, num, ni));
 #pragma unroll
                         for (int a = 0; a < NA; ++a)
-                            if (a == wi) sb[a] += worstBar / sAsset[a];
+                            if (a == wi) sb[a] += over(worstBar, sAsset[a], F32 ? Real(0) : sInv[a]);
                     }
                 }
                 // undo step i, asset by asset (assets are coupled only through the Gaussians)
@@ -351,7 +382,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 || sizeof(Real) == 4 ? 1 : RN
                     }
                     else
                     {
-                        const Real E = exp(dr + sd * cw);
+                        const Real E = exp_fx(p.fx, dr + sd * cw);
                         const Real base = dy == MD_LOGNORMAL ? fwd : dy == MD_SURNORMAL ? fwd + al : fwd - al;
                         const Real ub = abar * base * E;
                         fwdBar = abar * E;

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(MC_BLOCK) multi_kernel(const MultiParams mp)
                     }
                     else
                     {
-                        x[a] = x[a] * exp(bs[s] + bs[nSteps + s] * ga);
+                        x[a] = x[a] * exp_fx(p.fx, bs[s] + bs[nSteps + s] * ga);
                         tv[a] += bs[4 * nSteps + s] + bs[3 * nSteps + s] * ga;
                         tr[a] += bs[2 * nSteps + s];
                     }

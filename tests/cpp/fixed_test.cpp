@@ -219,6 +219,30 @@ static int smoothing()
     return bad != 0;
 }
 
+// Relative error: 2^-56 for the sum of the roundings, and the argument's own unit.
+static int exponential()
+{
+    std::vector<long long> t(1 << cf::FX_EXP_BITS);
+    cf::exp_table64(t.data());
+    std::mt19937_64 g(9);
+    long bad = 0;
+    auto check = [&](long long a) {
+        int n;
+        const long long m = cf::fx_exp(t.data(), a, n);
+        const real ref = expl(ldexpl((real)a, -cf::FX_A));
+        if (m < (1LL << 60) || !(fabsl(ldexpl((real)m, n - 61) / ref - 1.0L) <= ldexpl(1.0L, -56))) ++bad;
+    };
+    for (int i = 0; i < 300000; ++i) check((long long)(g() >> (1 + g() % 60)) * ((i & 1) ? 1 : -1) % (1LL << 62));
+    for (int i = -2000; i <= 2000; ++i)  // around the table's steps
+    {
+        const long long a = llrintl(ldexpl(i * logl(2.0L) / 256, cf::FX_A));
+        check(a), check(a + 1), check(a - 1);
+    }
+    check(0), check((1LL << 62) - 1), check(-(1LL << 62) + 1);
+    std::printf("%s exponential\n", bad ? "BAD" : "ok");
+    return bad != 0;
+}
+
 int main()
 {
     auto even = [](double a, double b, int n) {
@@ -228,7 +252,7 @@ int main()
     };
     std::vector<double> uneven;
     for (int i = 0; i < 40; ++i) uneven.push_back(40.0 + 3.0 * i + (i % 7 == 0 ? 0.02 : 1.1));
-    int bad = split() + gauss(0) + gauss(1) + gauss(2) + smoothing();
+    int bad = split() + gauss(0) + gauss(1) + gauss(2) + smoothing() + exponential();
     bad += paths("60 knots", 100.0, even(50, 200, 60), 156, 0.2, 300, true);
     bad += paths("120 knots, 520 steps", 100.0, even(50, 200, 120), 520, 0.3, 100, true);
     bad += paths("uneven knots", 100.0, uneven, 36, 0.25, 300, true);

@@ -70,8 +70,8 @@ CF_HD long long fx_mul32(long long s, int w)
 // ---------------------------------------------------------------------------------------
 constexpr int FX_Y = 57, FX_V = 62, FX_G = 59;
 // A bucket is no wider than the smallest gap between knots, so it holds at most one.  Its entry is
-// the first knot above its left edge with the number of knots up to the edge in the low bits (the
-// knot moves by less than 2^-40 for it; the vol is continuous there).
+// the first knot above its left edge with the number of knots up to the edge in the low bits (for
+// that it moves down by less than 2^13 units; the vol is continuous there).
 constexpr int FX_LO_BITS = 12;
 struct alignas(16) FxInterval  // between knots lo - 1 and lo; the flat ends have all zero
 {

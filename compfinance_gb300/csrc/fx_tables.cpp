@@ -40,7 +40,8 @@ int lower_with(const FxInput& in, double reach, int r, FxHost& h)
     for (long long b = 0; b < nB; ++b)
     {
         const int lo = int(std::upper_bound(K.begin(), K.end(), x0 + (b << wb)) - K.begin());
-        h.bucket.push_back(((lo < nS ? K[lo] : INT64_MAX) & ~loMask) | lo);
+        // at most the knot: a state on it (today's spot, often) belongs to the interval above
+        h.bucket.push_back((((lo < nS ? K[lo] : INT64_MAX) - loMask) & ~loMask) | lo);
     }
     const double most = std::ldexp(0.999, 62);  // of a vol; slopes and D may use another bit
     h.center = (K[0] + K[nS - 1]) / 2;

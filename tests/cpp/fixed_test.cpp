@@ -157,10 +157,10 @@ static int paths(const char* what, double spot, std::vector<double> spots, int s
         return lo;
     };
     for (int j = 0; j < nS; ++j)
-        for (long long d : {-5000LL, 5000LL, 1LL << 40, -(1LL << 40)})
+        for (long long d : {0LL, 5000LL, -9000LL, 1LL << 40, -(1LL << 40)})
         {
             const long long y = llrintl(in.X[j] / unitY) + d;
-            if (interval(y) != where(y)) ++bad;
+            if (interval(y) != (d == 0 ? j + 1 : where(y))) ++bad;
         }
     real worst = 0.0L, bound = 0.0L;
     for (int k = 0; k < paths; ++k)

@@ -19,6 +19,8 @@ def _grid(name):
     rs = np.random.RandomState(3)
     if name == "uneven":
         s, t = np.cumsum(rs.uniform(0.05, 6.0, 40)) + 40.0, np.array([0.2, 0.21, 1.0, 2.9])
+    elif name == "on_knot":
+        s, t = np.array([50.0, 80.0, 100.0, 120.0, 170.0]), np.array([0.5, 1.0, 2.0])
     elif name == "one_knot":
         s, t = np.array([90.0]), np.array([0.5, 2.0])
     else:
@@ -56,6 +58,7 @@ CASES = [
     ("60", 150.0, _uoc(), 500, 1, (1, 1)),               # knocked out today
     ("60", 100.0, _uoc(smooth=0.0005), 4000, 0, (1, 0)),  # adjoints beyond the slab's range
     ("uneven", 100.0, _uoc(), 2000, 0, (1, 0)),
+    ("on_knot", 100.0, _uoc(), 2000, 0, (1, 0)),         # today's spot on a knot: the interval above it
     ("one_knot", 100.0, _uoc(), 2000, 1, (1, 0)),
     ("60", 1.5, _uoc(barrier=2.1, strike=1.5), 500, 0, (1, 0)),  # far below the grid
     ("20_high", 100.0, _uoc(12), 2000, 0, (1, 0)),

@@ -606,11 +606,12 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
             oTd = pk.vec(tdv);
             oBf = pk.vec(bf);
         }
-        // a European's or barrier's last date is maturity, and a European has no other
+        // fixed-point FP64 form (dupire_fx64, multi_risk64.cu): a European's or barrier's last date is
+        // maturity, and a European has no other; portfolios may have any dates
         bool endOk = evAtStep[n] == plan.nEv - 1;
         if (pd.kind == PROD_EUROPEAN)
             for (int i = 0; i < n; ++i) endOk = endOk && evAtStep[i] < 0;
-        if ((pd.kind == PROD_UOC || pd.kind == PROD_EUROPEAN) && endOk)
+        if (((pd.kind == PROD_UOC || pd.kind == PROD_EUROPEAN) && endOk) || pd.kind == PROD_EUROPEANS)
         {
             plan.fxState = 0;
             FxInput& in = plan.fxIn;
@@ -870,7 +871,7 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     // FP64 Dupire European and barrier runs in fixed point at every size their tables fit: 60x30 weekly
     // barrier risk 9.5 -> 0.62 ms at 2^18 paths (141 -> 5.6 ms at 2^22), its value 5.2 -> 0.30 ms,
     // 20x10 grid and 10^5 x 52 steps 0.85 -> 0.14 ms against the generic kernel
-    if (!fp32 && !generic && fxReady(plan))
+    if (!fp32 && !generic && plan.prod != PROD_EUROPEANS && fxReady(plan))
     {
         p.fx = plan.fx;
         setGenerator(p, sobol);
@@ -1031,9 +1032,12 @@ size_t Context::footprint(const Plan& plan, const cf_num_param& num, bool risk, 
                size_t(plan.nPay + plan.nEv) * size_t(plan.nParam) * 16 + size_t(plan.nPay) * size_t(plan.nParam) * 8 +
                size_t(plan.nPay + plan.nEv) * 96 + 8192;
     }
+    if (plan.prod == PROD_EUROPEANS && risk && !generic && plan.fxState >= 0 && multi64Fits(plan, num))
+        return multi64Bytes(plan, num) + size_t(plan.nPay + plan.nEv) * size_t(plan.nParam) * 16 +
+               size_t(plan.nPay) * size_t(plan.nParam) * 8 + size_t(plan.nPay + plan.nEv) * 104 + 8192;
     const int fields = plan.prod == PROD_EUROPEANS ? 1 + 3 * NP : mc_scratch_fields(l, mc_rounds(l, num.numPath, threads));
     size_t b = size_t(plan.nParam + 2 * plan.nPay + 2) * 16 + size_t(plan.nPay) * 12 + 4096;
-    if (risk && !fp32 && !generic && plan.fxState >= 0)
+    if (risk && !fp32 && !generic && plan.fxState >= 0 && plan.prod != PROD_EUROPEANS)
     {
         // dupire_fx64: at most 7 blocks of 128 or 2 of 384 threads per SM, a ring of round slots
         l.fast = 3;

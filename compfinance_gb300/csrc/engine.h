@@ -222,10 +222,13 @@ struct Context
     // AADriskMulti: the multi kernel (European portfolios) is asynchronous like enqueue
     bool multiFast(const Plan& plan) const;
     bool multi32Use(const Plan& plan, const cf_num_param& num) const;  // FP32 Dupire: multi_risk32.cu
+    bool multi64Fits(const Plan& plan, const cf_num_param& num) const;  // FP64 Dupire: multi_risk64.cu, if fxReady
+    size_t multi64Bytes(const Plan& plan, const cf_num_param& num) const;  // its scratch
     // directRisks: the caller's nParam x nPay array, written before the call returns; aggWeights
     // (nPay): the run's risks are those of the weighted sum of the payoffs (nParam values)
+    // generic: FP64 in double arithmetic (multi_kernel.cu: little scratch)
     int enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, double* directRisks = nullptr,
-                     const double* aggWeights = nullptr);
+                     const double* aggWeights = nullptr, bool generic = false);
     int finishMulti(Slot& slot, double* values, double* risks, double* aggregate = nullptr);
     // AADriskOne / AADriskAggregate on the main slot: values, aggregate and risks of sum_k w_k payoff_k
     int aggregateRisk(Plan& plan, const cf_num_param& num, const double* weights, double* values, double* aggregate,

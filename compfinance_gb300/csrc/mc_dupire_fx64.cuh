@@ -23,7 +23,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include "cf_device.cuh"
+#include "fx_device.cuh"
 
 namespace cf {
 
@@ -269,23 +269,6 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
             double ax = __longlong_as_double(ey[seedRow]);
             double aAl = UOC ? __longlong_as_double(eb[seedRow]) : 0.0;
             ax *= 0x1p-59;  // carried in the Gaussians' unit
-            // v 2^sft, rounded, into a 96-bit word of 2^-60
-            auto nodeAdd = [&](int i, long long v, int sft) {
-                if (sft < 0)
-                {
-                    v = sft < -62 ? 0 : (v + (1LL << (-sft - 1))) >> -sft;
-                    sft = 0;
-                }
-                const unsigned l = (unsigned)v, h = (unsigned)((unsigned long long)v >> 32);
-                const unsigned a0 = l << sft, a1 = __funnelshift_l(l, h, sft);
-                unsigned a2 = (unsigned)((int)h >> (sft ? 32 - sft : 31));
-                unsigned* at = node + i;
-                const unsigned o0 = atomicAdd(at, a0), c0 = o0 + a0 < o0 ? 1u : 0u;
-                const unsigned o1 = atomicAdd(at + nNodes, a1 + c0);
-                // a1 + c0 wraps to 0 only with a carry of its own
-                a2 += (a1 + c0 < c0 ? 1u : 0u) + (o1 + (a1 + c0) < o1 ? 1u : 0u);
-                if (a2) atomicAdd(at + 2 * nNodes, a2);
-            };
             // states and Gaussians are loaded two steps ahead
             long long yA = __ldcs(ey + (nSteps - 1) * Ti), gA = __ldcs(es + (nSteps - 1) * Ti), yB = 0, gB = 0;
             if (nSteps >= 2)
@@ -307,46 +290,7 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
                 const long long v = volAt(s, y, lo);
                 const double av = ax * (double)(g - 2 * (v >> (4 - r)));  // d y_{s+1} / d v = g - v
                 ax = fma(av, __ldg(p.fx.slope + s * pitch + lo), ax);
-                if (av != 0.0)
-                {
-                    const FxInterval iv = sIv[lo];
-                    const bool inner = lo > 0 && lo < nS;  // two knots; one at the flat ends
-                    const long long t =
-                        inner ? fx_mul_add(sInv[lo], (long long)((unsigned long long)(y - iv.x) << iv.sh), 0) : 0;
-                    const int jl = lo - (lo > 0 ? 1 : 0);
-                    const longlong2 s0 = __ldg(reinterpret_cast<const longlong2*>(p.fx.step + s));
-                    const int2 col = __ldg(reinterpret_cast<const int2*>(&p.fx.step[s].colA));
-                    // the adjoint of sigma as N 2^sft units of 2^-60: its 53-bit mantissa
-                    const double c = av * __longlong_as_double(s0.y);
-                    const int hi = __double2hiint(c), E = (hi >> 20) & 0x7ff;
-                    const int sft = E - (1023 - FIX_LO_SHIFT + 52);
-                    if (sft <= p.fx.nodeShift)
-                    {
-                        const unsigned long long m = ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32) |
-                                               (unsigned)__double2loint(c);
-                        const long long N = hi < 0 ? -(long long)m : (long long)m;
-                        const long long nR = fx_mul_add(N * 32, t, 0), nL = N - nR;
-                        const long long rB = fx_mul_add(nR * 4, s0.x, 0), lB = fx_mul_add(nL * 4, s0.x, 0);
-                        const int at = jl * nT;
-                        nodeAdd(at + col.x, nL - lB, sft);
-                        nodeAdd(at + col.y, lB, sft);
-                        if (inner)
-                        {
-                            nodeAdd(at + nT + col.x, nR - rB, sft);
-                            nodeAdd(at + nT + col.y, rB, sft);
-                        }
-                    }
-                    else
-                    {
-                        const double cR = c * ((double)t * 0x1p-59), cL = c - cR;
-                        const double tw = (double)s0.x * 0x1p-62;
-                        long long* acc = p.acc + 2 * (1 + jl * nT);
-                        fix_add(acc + 2 * col.x, cL - cL * tw);
-                        fix_add(acc + 2 * col.y, cL * tw);
-                        fix_add(acc + 2 * (nT + col.x), cR - cR * tw);  // cR = 0 at the flat ends
-                        fix_add(acc + 2 * (nT + col.y), cR * tw);
-                    }
-                }
+                if (av != 0.0) fx_vol_adjoint(p, p.acc, node, nNodes, sIv, sInv, s, lo, y, av);
                 // the date at point s: survival below the barrier's smoothing band
                 if (UOC && y > yBand && aAl != 0.0 && (evEvery ? s > 0 || p.evAtStep[0] >= 0 : __ldg(p.evAtStep + s) >= 0))
                 {
@@ -360,18 +304,7 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
         }
         head += n;
         __syncthreads();
-        for (int i = tid; i < nNodes; i += RB)
-        {
-            const unsigned n0 = node[i], n1 = node[i + nNodes], n2 = node[i + 2 * nNodes];
-            if (n0 | n1 | n2)
-            {
-                node[i] = node[i + nNodes] = node[i + 2 * nNodes] = 0;
-                const long long lo = (long long)(((unsigned long long)(n1 & 0xffu) << 32) | n0);  // 40 bits
-                const long long hi = (long long)(((unsigned long long)n2 << 32) | n1) >> 8;
-                if (hi) atomicAdd(reinterpret_cast<unsigned long long*>(&p.acc[2 * (1 + i)]), (unsigned long long)hi);
-                if (lo) atomicAdd(reinterpret_cast<unsigned long long*>(&p.acc[2 * (1 + i) + 1]), (unsigned long long)lo);
-            }
-        }
+        fx_node_flush(p.acc, node, nNodes, RB);
         __syncthreads();
     };
 

@@ -7,6 +7,8 @@
 // suffix sums (multi_finish).  Other products (one or two payoffs) run one adjoint sweep per
 // payoff over the same random numbers; both give the exact per-payoff path averages.
 #include <algorithm>
+#include <cmath>
+#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
@@ -34,6 +36,8 @@ int launch_multi_aggregate(const double* risks, int nParam, int nPay, const doub
 int launch_multi_finish(const long long* accR, int nAccParam, int nOut, int nEv, const int* evOff, const double* ks,
                         const int* orig, int nPay, int bs, double n, double* risks, void* stream);
 
+int fx_node_shift(const Plan& plan, int block);  // fx_plan.cpp
+
 constexpr int kMultiMaxE = 16;
 
 const ProductDesc* Context::productOf(const Plan& plan) const
@@ -49,7 +53,7 @@ bool Context::multiFast(const Plan& plan) const
 }
 
 int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, double* directRisks,
-                          const double* aggWeights)
+                          const double* aggWeights, bool generic)
 {
     const ProductDesc* pd = productOf(plan);
     if (!multiFast(plan)) return fail(CF_E_UNSUPPORTED, "multi kernel: European portfolios of <= 16 maturities");
@@ -78,13 +82,21 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
     const int nBuckets = slot.evOff[nEv];
     const int nParam = plan.model == MODEL_BS ? 8 : plan.nParam;  // BS: (a, b) per parameter
     const bool fast = multi32Use(plan, num);
+    const bool fx = !fp32 && !generic && multi64Fits(plan, num) && fxReady(plan);
     std::vector<float> ksf(slot.ks.begin(), slot.ks.end());
+    std::vector<long long> ksi;  // fixed-point form: the last state at which the spot is not above the strike
+    if (fx)
+        for (double k : slot.ks)
+        {
+            const double x = k > 0.0 ? std::floor(std::ldexp(std::log(k) - plan.base.x0d, FX_Y - plan.fx.r)) : -INFINITY;
+            ksi.push_back(!(x > -9.2e18) ? INT64_MIN : x < 9.2e18 ? (long long)x : INT64_MAX);
+        }
     // device buffer: inputs (bucket offsets, strikes, payoff index per sorted strike), the
     // zeroed accumulators and counters, the bucket segments of the FP32 kernels, the risks
     auto up = [](size_t n) { return 256 * ((n + 255) / 256); };
     const size_t offKs = up(slot.evOff.size() * 4);
     const size_t offKsf = offKs + up(slot.ks.size() * 8);
-    const size_t offOrig = offKsf + up(ksf.size() * 4);
+    const size_t offOrig = offKsf + up(ksf.size() * 8);  // FP32 strikes, or the fixed-point ones
     const size_t offAccR = offOrig + up(slot.orig.size() * 4);
     const size_t accRBytes = size_t(nBuckets) * nParam * 16;
     slot.accVBytes = size_t(nBuckets) * 5 * 16;
@@ -107,20 +119,22 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
     slot.aggW.assign(aggWeights ? aggWeights : nullptr, aggWeights ? aggWeights + plan.nPay : nullptr);
     slot.accRBytes = aggWeights ? size_t(plan.nParam) * 8 : directRisks ? 0 : riskBytes;
     if ((rc = slot.hostAcc.ensure(slot.accRBytes + slot.accVBytes + 16))) return rc;
-    const size_t wBytes = slot.evOff.size() * 4 + slot.ks.size() * 12 + slot.orig.size() * 4;
+    const size_t offB = (slot.evOff.size() * 4 + 7) & ~size_t(7);  // 8-byte aligned strikes
+    const size_t wBytes = (offB + slot.ks.size() * 16 + slot.orig.size() * 4 + 7) & ~size_t(7);
     if ((rc = slot.hostW.ensure(wBytes + size_t(plan.nPay) * 8 + 64))) return rc;
     char* hw = static_cast<char*>(slot.hostW.ptr);
-    char* hKs = hw + slot.evOff.size() * 4;
+    char* hKs = hw + offB;
     char* hKsf = hKs + slot.ks.size() * 8;
-    char* hOrig = hKsf + ksf.size() * 4;
+    char* hOrig = hKsf + ksf.size() * 8;
     std::memcpy(hw, slot.evOff.data(), slot.evOff.size() * 4);
     std::memcpy(hKs, slot.ks.data(), slot.ks.size() * 8);
-    std::memcpy(hKsf, ksf.data(), ksf.size() * 4);
+    if (fx) std::memcpy(hKsf, ksi.data(), ksi.size() * 8);
+    else std::memcpy(hKsf, ksf.data(), ksf.size() * 4);
     std::memcpy(hOrig, slot.orig.data(), slot.orig.size() * 4);
     char* d = static_cast<char*>(slot.multiBuf.ptr);
     cudaError_t e = cudaMemcpyAsync(d, hw, slot.evOff.size() * 4, cudaMemcpyHostToDevice, st);
     if (!e) e = cudaMemcpyAsync(d + offKs, hKs, slot.ks.size() * 8, cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemcpyAsync(d + offKsf, hKsf, ksf.size() * 4, cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaMemcpyAsync(d + offKsf, hKsf, ksf.size() * (fx ? 8 : 4), cudaMemcpyHostToDevice, st);
     if (!e) e = cudaMemcpyAsync(d + offOrig, hOrig, slot.orig.size() * 4, cudaMemcpyHostToDevice, st);
     if (!e) e = cudaMemsetAsync(d + offAccR, 0, zeroEnd - offAccR, st);
     if (!e && aggWeights)
@@ -142,10 +156,10 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
     const int* dEvOff = reinterpret_cast<const int*>(d);
     long long* dAccR = reinterpret_cast<long long*>(d + offAccR);
     long long* dAccV = reinterpret_cast<long long*>(d + offAccV);
-    if (fast)
+    if (fast || fx)
     {
-        // FP32 Dupire: forward, bucket segments, chunked reverse sweeps (multi_risk32.cu)
-        Multi32Args A;
+        // Dupire: forward, bucket segments, chunked reverse sweeps (multi_risk32.cu, multi_risk64.cu)
+        Multi32Args A{};
         A.p = p;
         A.nParam = nParam;
         A.nBuckets = nBuckets;
@@ -161,21 +175,46 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
         A.chunkStart = reinterpret_cast<int*>(d + offChunk);
         A.work = reinterpret_cast<int*>(d + offErr + 16);
         const size_t nP = size_t(num.numPath), nE = size_t(nEv);
-        const size_t recBytes = up(nP * A.pitch * 8), evBBytes = up(nE * nP * 2), evSBytes = up(nE * nP * 4);
-        if ((rc = slot.scratch.ensure(recBytes + evBBytes + evSBytes + nE * nP * 8, st))) return rc;
-        char* sc = static_cast<char*>(slot.scratch.ptr);
-        A.rec = reinterpret_cast<unsigned*>(sc);
-        A.evB = reinterpret_cast<unsigned short*>(sc + recBytes);
-        A.evS = reinterpret_cast<float*>(sc + recBytes + evBBytes);
-        A.list = reinterpret_cast<int*>(sc + recBytes + evBBytes + evSBytes);
-        const size_t smemF = m32_forward_smem(sobol, A), smemR = m32_reverse_smem(A);
-        int occF = 0, occR = 0;
-        rc = m32_occupancy(sobol, smemF, smemR, &occF, &occR);
-        if (rc) return cuda_fail(cudaError_t(rc), "multi occupancy");
-        if (occF < 1 || occR < 1) return fail(CF_E_SHAPE, "multi kernel does not fit on an SM");
         const long long threadsNeeded = sobol ? (p.nPath / 32 + 1) * 32 : (p.nPath + 1) / 2;
-        const long long gridF = std::max(1LL, std::min<long long>((threadsNeeded + 127) / 128, (long long)numSMs * occF));
-        rc = launch_multi32(sobol, int(gridF), smemF, numSMs * occR, smemR, A, st);
+        int occF = 0, occR = 0;
+        if (fx)
+        {
+            A.p.fx = plan.fx;
+            setGenerator(A.p, sobol);
+            A.p.fx.nodeShift = fx_node_shift(plan, M32_CHUNK);
+            A.ksI = reinterpret_cast<const long long*>(d + offKsf);
+            const size_t recBytes = up(nP * plan.nSteps * 16), evBBytes = up(nE * nP * 2), evSBytes = up(nE * nP * 8);
+            rc = slot.scratch.ensure(multi64Bytes(plan, num), st);
+            if (rc == CF_E_NOMEM) return enqueueMulti(slot, plan, num, directRisks, aggWeights, true);
+            if (rc) return rc;
+            char* sc = static_cast<char*>(slot.scratch.ptr);
+            A.rec64 = reinterpret_cast<longlong2*>(sc);
+            A.evB = reinterpret_cast<unsigned short*>(sc + recBytes);
+            A.evS64 = reinterpret_cast<double*>(sc + recBytes + evBBytes);
+            A.list64 = reinterpret_cast<longlong2*>(sc + recBytes + evBBytes + evSBytes);
+            const size_t smemF = m64_forward_smem(sobol, A), smemR = m64_reverse_smem(A);
+            rc = smemF > 227 * 1024 || smemR > 227 * 1024 ? 0 : m64_occupancy(sobol, smemF, smemR, &occF, &occR);
+            if (rc) return cuda_fail(cudaError_t(rc), "multi occupancy");
+            if (occF < 1 || occR < 1) return enqueueMulti(slot, plan, num, directRisks, aggWeights, true);
+            const long long gridF = std::max(1LL, std::min<long long>((threadsNeeded + 127) / 128, (long long)numSMs * occF));
+            rc = launch_multi64(sobol, int(gridF), smemF, numSMs * occR, smemR, A, st);
+        }
+        else
+        {
+            const size_t recBytes = up(nP * A.pitch * 8), evBBytes = up(nE * nP * 2), evSBytes = up(nE * nP * 4);
+            if ((rc = slot.scratch.ensure(recBytes + evBBytes + evSBytes + nE * nP * 8, st))) return rc;
+            char* sc = static_cast<char*>(slot.scratch.ptr);
+            A.rec = reinterpret_cast<unsigned*>(sc);
+            A.evB = reinterpret_cast<unsigned short*>(sc + recBytes);
+            A.evS = reinterpret_cast<float*>(sc + recBytes + evBBytes);
+            A.list = reinterpret_cast<int*>(sc + recBytes + evBBytes + evSBytes);
+            const size_t smemF = m32_forward_smem(sobol, A), smemR = m32_reverse_smem(A);
+            rc = m32_occupancy(sobol, smemF, smemR, &occF, &occR);
+            if (rc) return cuda_fail(cudaError_t(rc), "multi occupancy");
+            if (occF < 1 || occR < 1) return fail(CF_E_SHAPE, "multi kernel does not fit on an SM");
+            const long long gridF = std::max(1LL, std::min<long long>((threadsNeeded + 127) / 128, (long long)numSMs * occF));
+            rc = launch_multi32(sobol, int(gridF), smemF, numSMs * occR, smemR, A, st);
+        }
         if (rc) return cuda_fail(cudaError_t(rc), "multi kernel launch");
         slot.launches = 5;
     }
@@ -249,6 +288,21 @@ bool Context::multi32Use(const Plan& plan, const cf_num_param& num) const
     return !(env && env[0] == '0');
 }
 
+// FP64 Dupire portfolios in fixed point: list positions are int32, and the records (16 bytes per path
+// and step) are held to 32 GB; beyond, and for models outside the fixed-point ranges, multi_kernel.
+bool Context::multi64Fits(const Plan& plan, const cf_num_param& num) const
+{
+    return plan.model == MODEL_DUPIRE && plan.prod == PROD_EUROPEANS && num.precision != CF_FP32 && num.numPath > 0 &&
+           (long long)plan.nEv * num.numPath < (1LL << 30) && multi64Bytes(plan, num) <= (size_t(32) << 30);
+}
+
+size_t Context::multi64Bytes(const Plan& plan, const cf_num_param& num) const
+{
+    const size_t nP = size_t(num.numPath), nE = size_t(plan.nEv);
+    auto up = [](size_t n) { return 256 * ((n + 255) / 256); };
+    return up(nP * plan.nSteps * 16) + up(nE * nP * 2) + up(nE * nP * 8) + nE * nP * 16;
+}
+
 int Context::finishMulti(Slot& slot, double* values, double* risks, double* aggregate)
 {
     const Plan& plan = *slot.plan;
@@ -298,10 +352,10 @@ int Context::aggregateRisk(Plan& plan, const cf_num_param& num, const double* we
                            double* aggregate, double* risks)
 {
     main.stream = stream;
-    // FP32 European portfolios on Dupire: the portfolio kernels (every payoff's risks, then their
-    // weighted sum on the device) take the work in a fraction of the time of one aggregated
-    // adjoint through the generic kernel; the risks are the same linear functional of the paths
-    if (multiFast(plan) && multi32Use(plan, num))
+    // European portfolios on Dupire: the portfolio kernels (every payoff's risks, then their weighted
+    // sum on the device) take the work in a fraction of the time of one aggregated adjoint through
+    // the generic kernel; the risks are the same linear functional of the paths
+    if (multiFast(plan) && (multi32Use(plan, num) || (multi64Fits(plan, num) && fxReady(plan))))
     {
         int rc = enqueueMulti(main, plan, num, nullptr, weights);
         if (rc) return rc;

@@ -1,5 +1,5 @@
-// FP32 AADriskMulti of a European portfolio on the Dupire model (multi_risk32.cu): launch
-// arguments shared by the host (multi.cpp) and the kernels.
+// AADriskMulti of a European portfolio on the Dupire model (multi_risk32.cu, and its FP64 form
+// multi_risk64.cu): launch arguments shared by the host (multi.cpp) and the kernels.
 #pragma once
 #include <cstddef>
 
@@ -29,6 +29,11 @@ struct Multi32Args
     int* chunkStart;       // [nBuckets+1] first chunk of each bucket; [nBuckets] = chunks
     int* work;             // reverse chunk counter (zeroed)
     int* list;             // [2 * entries]: path, spot bits; grouped by bucket
+    // FP64 form
+    const long long* ksI;  // [nKs] state above which the spot is above the strike, order of ksF
+    longlong2* rec64;      // [nPath][nSteps]: state, Gaussian (the path's own sign)
+    double* evS64;         // [nEv][nPath] spot at maturity e
+    longlong2* list64;     // [entries]: path, spot bits
 };
 
 size_t m32_forward_smem(int rng, const Multi32Args& a);
@@ -36,7 +41,17 @@ size_t m32_reverse_smem(const Multi32Args& a);
 // occupancy (blocks per SM) of the forward and reverse kernels for these shared-memory sizes
 int m32_occupancy(int rng, size_t smemFwd, size_t smemRev, int* occFwd, int* occRev);
 // forward, scan, scatter and reverse on one stream; returns cudaError_t
+int launch_multi32_scan(const Multi32Args& a, void* stream);
+int launch_multi32_scatter(const Multi32Args& a, bool f64, void* stream);
 int launch_multi32(int rng, int gridFwd, size_t smemFwd, int gridRev, size_t smemRev, const Multi32Args& a,
+                   void* stream);
+
+// FP64 form in fixed point
+constexpr int M64_BLOCK = 256;  // threads of a reverse block: one per entry of a chunk
+size_t m64_forward_smem(int rng, const Multi32Args& a);
+size_t m64_reverse_smem(const Multi32Args& a);
+int m64_occupancy(int rng, size_t smemFwd, size_t smemRev, int* occFwd, int* occRev);
+int launch_multi64(int rng, int gridFwd, size_t smemFwd, int gridRev, size_t smemRev, const Multi32Args& a,
                    void* stream);
 
 }  // namespace cf

@@ -328,6 +328,7 @@ __global__ void multi32_scan(const Multi32Args A)
 // ---------------------------------------------------------------------------------------
 constexpr int SC_BLOCK = 256, SC_ITEMS = 8, SC_PER = SC_BLOCK * SC_ITEMS;
 
+template <bool F64>
 __global__ void __launch_bounds__(SC_BLOCK) multi32_scatter(const Multi32Args A)
 {
     extern __shared__ int sCount[];  // [nBuckets]: block counts, then the block's global offsets
@@ -366,8 +367,14 @@ __global__ void __launch_bounds__(SC_BLOCK) multi32_scatter(const Multi32Args A)
         {
             const long long i = i0 + j * SC_BLOCK + tid;
             const int at = sCount[bk[j]] + rank[j];
-            A.list[2 * at] = int(i - (i / nPath) * nPath);
-            A.list[2 * at + 1] = __float_as_int(A.evS[i]);
+            const int path = int(i - (i / nPath) * nPath);
+            if (F64)
+                A.list64[at] = make_longlong2(path, __double_as_longlong(A.evS64[i]));
+            else
+            {
+                A.list[2 * at] = path;
+                A.list[2 * at + 1] = __float_as_int(A.evS[i]);
+            }
         }
 }
 
@@ -534,6 +541,23 @@ int m32_occupancy(int rng, size_t smemFwd, size_t smemRev, int* occFwd, int* occ
     return (int)e;
 }
 
+int launch_multi32_scan(const Multi32Args& a, void* stream)
+{
+    Multi32Args q = a;
+    void* args[] = {&q};
+    return (int)cudaLaunchKernel((const void*)&multi32_scan, dim3(1), dim3(32), args, 0, (cudaStream_t)stream);
+}
+
+int launch_multi32_scatter(const Multi32Args& a, bool f64, void* stream)
+{
+    Multi32Args q = a;
+    void* args[] = {&q};
+    const long long total = (long long)a.p.nEv * a.p.nPath;
+    return (int)cudaLaunchKernel(f64 ? (const void*)&multi32_scatter<true> : (const void*)&multi32_scatter<false>,
+                                 dim3(unsigned((total + SC_PER - 1) / SC_PER)), dim3(SC_BLOCK), args,
+                                 size_t(a.nBuckets) * 4, (cudaStream_t)stream);
+}
+
 int launch_multi32(int rng, int gridFwd, size_t smemFwd, int gridRev, size_t smemRev, const Multi32Args& a,
                    void* stream)
 {
@@ -541,11 +565,8 @@ int launch_multi32(int rng, int gridFwd, size_t smemFwd, int gridRev, size_t sme
     Multi32Args q = a;
     void* args[] = {&q};
     cudaError_t e = cudaLaunchKernel(fwd_ptr(rng), dim3(gridFwd), dim3(MB), args, smemFwd, st);
-    if (!e) e = cudaLaunchKernel((const void*)&multi32_scan, dim3(1), dim3(32), args, 0, st);
-    const long long total = (long long)a.p.nEv * a.p.nPath;
-    if (!e)
-        e = cudaLaunchKernel((const void*)&multi32_scatter, dim3(unsigned((total + SC_PER - 1) / SC_PER)),
-                             dim3(SC_BLOCK), args, size_t(a.nBuckets) * 4, st);
+    if (!e) e = (cudaError_t)launch_multi32_scan(a, stream);
+    if (!e) e = (cudaError_t)launch_multi32_scatter(a, false, stream);
     if (!e) e = cudaLaunchKernel((const void*)&multi32_reverse, dim3(gridRev), dim3(MB), args, smemRev, st);
     return (int)e;
 }

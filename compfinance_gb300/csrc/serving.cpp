@@ -93,7 +93,7 @@ public:
         {
             r.nPay = plan->nPay;
             r.nParam = plan->nParam;
-            if (r.kind == 2) rc = c.enqueueMulti(*slots[s], *plan, r.num);
+            if (r.kind == 2) rc = c.enqueueMulti(*slots[s], *plan, r.num, nullptr, nullptr, r.generic);
             else
             {
                 if (r.kind == 1 && r.w.empty())
@@ -296,9 +296,9 @@ int cf_server_submit(cf_server* s, const cf_request* r, uint64_t* id)
     q.num = r->num;
     if (r->weights) q.w.assign(r->weights, r->weights + r->nWeights);
     size_t fp = s->ctx->c.footprint(*plan, r->num, r->kind != 0);
-    if (fp > s->sched.budget() && r->kind == 1)
+    if (fp > s->sched.budget() && r->kind != 0)
     {
-        // an FP64 risk whose ring of round slots exceeds the budget runs the generic kernel
+        // an FP64 risk whose fixed-point form's scratch exceeds the budget runs the generic kernel
         const size_t small = s->ctx->c.footprint(*plan, r->num, true, true);
         q.generic = small < fp;
         fp = std::min(fp, small);

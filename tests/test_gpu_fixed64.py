@@ -98,3 +98,47 @@ def test_value_and_risk_against_the_oracle(eng, k):
     assert np.array_equal(x["values"], r["payoffValues"])
     y = eng.simulatePaths("m", "p", num(sob, n))
     assert rel_to_max(y.mean(axis=0), values) <= tol * max(1.0, band) + 1e-14
+
+
+def _strikes(n, lo=70.0, hi=150.0):
+    return [lo + (hi - lo) * i / max(1, n - 1) for i in range(n)]
+
+
+PORTFOLIOS = [
+    # grid, spot, [(maturity, strikes)], paths, sobol
+    ("60", 100.0, [(0.5, _strikes(20)), (1.0, _strikes(20)), (3.0, _strikes(20))], 1, 1),
+    ("60", 100.0, [(0.5, _strikes(5)), (2.0, _strikes(3))], 31, 0),
+    ("60", 100.0, [(0.5, _strikes(5)), (2.0, _strikes(3))], 257, 0),
+    ("20", 100.0, [(0.25 * k, _strikes(4)) for k in range(1, 17)], 1025, 1),   # 16 maturities
+    ("120", 100.0, [(1.5, _strikes(40)), (3.0, _strikes(1))], 3000, 0),        # slab of 86 KB
+    ("on_knot", 100.0, [(1.0, [100.0, 100.0, 90.0, 1e-3, 1e4]), (2.0, [100.0])], 2000, 1),  # equal and extreme strikes
+    ("uneven", 100.0, [(0.01, [99.0, 101.0]), (0.02, [100.0])], 511, 1),
+    ("one_knot", 80.0, [(1.0, _strikes(6))], 600, 0),
+    ("20_beyond", 100.0, [(1.0, _strikes(3))], 300, 0),                        # multi_kernel
+]
+
+
+@pytest.mark.parametrize("k", range(len(PORTFOLIOS)))
+def test_portfolio_against_the_oracle(eng, k):
+    """Tolerance: as above; a payoff's relative error is that of the spot times spot / payoff, a node
+    weight's that of log S over the smallest gap between knots."""
+    grid, spot, book, n, sob = PORTFOLIOS[k]
+    s, t, v = _grid(grid)
+    mats = [m for m, ks in book for _ in ks]
+    strikes = [x for _, ks in book for x in ks]
+    eng.putDupire(spot, s, t, v, 0.25, "m")
+    eng.putEuropeans(mats, strikes, "p")
+    m = O.Model(dict(kind="dupire", spot=spot, spots=s, times=t, vols=v, maxdt=0.25))
+    p = O.Product(dict(kind="europeans", mats=mats, strikes=strikes))
+    npay, _, steps = O.shapes(m, p)
+    values, risks = O.risk_multi(m, p, sob, n)
+    tol = 4 * np.sqrt(steps + 1) * max(1.0, abs(np.log(spot))) * 2.0 ** -51
+    gap = np.diff(np.log(s)).min() if len(s) > 1 else 1.0
+    r = eng.AADriskMulti("m", "p", num(sob, n))
+    assert np.abs(r["values"] - values).max() <= tol * spot * 4
+    assert rel_to_max(r["risks"], risks) <= 2 * tol * (1 + 1 / gap)
+    # the weighted book through the same kernels
+    w = np.random.RandomState(1).uniform(-1, 2, npay)
+    a = eng.AADriskAggregate("m", "p", w, num(sob, n))
+    assert rel_to_max(a["risks"], r["risks"] @ w) <= 1e-12
+    assert abs(a["riskPayoffValue"] - r["values"] @ w) <= 1e-12 * np.abs(w) @ r["values"]

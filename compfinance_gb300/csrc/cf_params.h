@@ -257,6 +257,9 @@ struct McLaunch
 int launch_mc(const McLaunch& l, const McParams& p, void* stream);   // returns cudaError_t
 int mc_smem_bytes(const McLaunch& l, const McParams& p, int stageY, size_t* bytes);
 int mc_occupancy(const McLaunch& l, size_t smem, int* blocksPerSM);
+// Threads per block of dupire_risk32 (l.block: 128, or 256 when that keeps more threads resident and
+// the run fills the device): returns the unstaged kernel's blocks per SM, 0 when it does not fit.
+int r32_block(McLaunch& l, McParams& p, long long threadsNeeded, int numSMs);
 // dupire_risk32 staging (p.stageY: inverse-normal table in shared memory; p.rowChunk: local-vol
 // rows staged by bulk copies) that keeps occ0 blocks per SM; sets *smem, returns the occupancy.
 int r32_staging(McLaunch& l, McParams& p, int occ0, size_t* smem);

@@ -868,6 +868,8 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     int occ0 = 0, occ1 = 0;
     l.fast = mc_use_fast32(plan.base, plan.prod, l.fp32, l.risk);
     l.block = 128;
+    // threads for one unit each of n paths
+    auto needOf = [sobol](long long n) { return sobol ? (n / 32 + 1) * 32 : (n + 1) / 2; };
     // FP64 Dupire European and barrier runs in fixed point at every size their tables fit: 60x30 weekly
     // barrier risk 9.5 -> 0.62 ms at 2^18 paths (141 -> 5.6 ms at 2^22), its value 5.2 -> 0.30 ms,
     // 20x10 grid and 10^5 x 52 steps 0.85 -> 0.14 ms against the generic kernel
@@ -880,7 +882,7 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
         int best = 0, block = 128;
         for (int b : {128, 384})
         {
-            if (b > 128 && !risk) break;
+            if (b > 128 && (!risk || needOf(chunk) <= (long long)numSMs * best)) break;
             l.block = b;
             size_t n = 0;
             int occ = 0;
@@ -910,10 +912,8 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     {
         // the local-vol rows (bulk copies) and the inverse-normal table go to shared memory when
         // that costs no occupancy
-        p.stageY = 0;
-        p.rowChunk = 0;
-        mc_smem_bytes(l, p, 0, &smem0);
-        if (smem0 > 200 * 1024 || mc_occupancy(l, smem0, &occ0) || occ0 < 1) l.fast = 0;
+        occ0 = r32_block(l, p, generic ? 0 : needOf(chunk), numSMs);
+        if (occ0 < 1) l.fast = 0;
         else occ0 = r32_staging(l, p, occ0, &smem0);
     }
     if (!l.fast)
@@ -944,9 +944,9 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     // chunked runs: the grid and the scratch are sized for one chunk, the launches below cover
     // the whole run
     p.nPath = chunk;
-    const long long threadsNeeded = sobol ? (p.nPath / 32 + 1) * 32 : (p.nPath + 1) / 2;
+    const long long threadsNeeded = needOf(p.nPath);
     long long grid = (threadsNeeded + l.block - 1) / l.block;
-    const long long maxGrid = (long long)numSMs * (maxBlocksPerSM > 0 ? std::min(occ, maxBlocksPerSM) : occ);
+    const long long maxGrid = (long long)numSMs * (maxBlocksPerSM > 0 ? std::min(occ, std::max(1, maxBlocksPerSM * 128 / l.block)) : occ);
     if (grid > maxGrid) grid = maxGrid;
     if (grid < 1) grid = 1;
     l.grid = int(grid);
@@ -1018,11 +1018,17 @@ size_t Context::footprint(const Plan& plan, const cf_num_param& num, bool risk, 
     McLaunch l{plan.model, plan.prod, sobol ? RNG_SOBOL : RNG_MRG, fp32 ? 1 : 0, risk ? 1 : 0, 0, 0, 0, 0};
     l.fast = mc_use_fast32(plan.base, plan.prod, l.fp32, l.risk);
     size_t smem = 0;
-    mc_smem_bytes(l, p, 0, &smem);
     int occ = 16;
-    if (mc_occupancy(l, smem, &occ) || occ < 1) occ = 16;
     const long long needed = sobol ? (num.numPath / 32 + 1) * 32 : (num.numPath + 1) / 2;
-    const long long threads = std::min<long long>(needed, (long long)numSMs * occ * 128);
+    if (l.fast) occ = r32_block(l, p, generic ? 0 : needed, numSMs);
+    else
+    {
+        mc_smem_bytes(l, p, 0, &smem);
+        if (mc_occupancy(l, smem, &occ)) occ = 0;
+    }
+    if (occ < 1) occ = 16;
+    const int block = l.fast && l.block ? l.block : 128;
+    const long long threads = std::min<long long>((needed + block - 1) / block * block, (long long)numSMs * occ * block);
     if (plan.prod == PROD_EUROPEANS && risk && multi32Use(plan, num))
     {
         // multi_risk32.cu: step records per path, bucket and spot per (maturity, path), entry
@@ -1045,7 +1051,7 @@ size_t Context::footprint(const Plan& plan, const cf_num_param& num, bool risk, 
         return b + size_t(mc_scratch_fields(l, mc_rounds(l, num.numPath, t))) * size_t(plan.nSteps + 1) * size_t(t) * 8;
     }
     if (risk) b += size_t(fields) * size_t(plan.nSteps + 1) * size_t(threads) * (fp32 ? 4 : 8);
-    if (risk && l.fast) b += size_t((threads + 127) / 128) * size_t(plan.base.nS) * size_t(plan.base.nT) * 8 + 256;
+    if (risk && l.fast) b += size_t((threads + block - 1) / block) * size_t(plan.base.nS) * size_t(plan.base.nT) * 8 + 256;
     // multi: bucket accumulators plus the finished per-payoff risks
     if (plan.prod == PROD_EUROPEANS && risk) b += size_t(plan.nPay + plan.nEv) * size_t(plan.nParam) * 16 + size_t(plan.nPay) * size_t(plan.nParam) * 8;
     return b;

@@ -204,10 +204,10 @@ struct Context
     // payoffs [path][nPay].  chunkPaths > 0 (a multiple of 64): the run is launched as
     // consecutive path ranges of at most that many paths, each adding into the same exact
     // accumulators (bit-identical results), so that kernels of other streams get the device
-    // between them.  maxBlocksPerSM > 0 caps the launch's resident blocks per SM below the
-    // kernel's occupancy, leaving room on every SM for kernels of other streams.  generic: FP64
-    // Dupire runs in double arithmetic (finite differences by bumping, runs that must fit the
-    // smaller scratch).
+    // between them.  maxBlocksPerSM > 0 caps the launch's resident blocks (of 128 threads) per SM below the
+    // kernel's occupancy, leaving room on every SM for kernels of other streams.  generic: the
+    // form with the smaller scratch: FP64 Dupire runs in double arithmetic (also finite differences by
+    // bumping), FP32 risks in blocks of 128.
     int enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk, const double* weights,
                 long long firstPath = 0, double* pathOut = nullptr, long long chunkPaths = 0,
                 int maxBlocksPerSM = 0, bool generic = false);

@@ -41,8 +41,6 @@ namespace cf {
 
 namespace {
 
-constexpr int RB = 128;                 // threads per block
-constexpr int RW = RB / 32;             // warps per block
 constexpr int T_BITS = 22;              // interpolation weight bits of the packed step word
 constexpr unsigned T_MASK = (1u << T_BITS) - 1;
 constexpr unsigned BAND_BIT = 1u << T_BITS;
@@ -56,8 +54,8 @@ constexpr float T_MAX = 1.0f - 1.0f / 4194304.0f;  // t + 2 stays below 3
 // nodeShiftF assumes this bound).  After a path passes through the barrier's smoothing band
 // its state adjoint is of the order of the spot over the band width, so this is common.
 constexpr float AV_MAX = 512.0f;
-// pending-path list: a power of two above the most it holds (127 left over + 2 RB new)
-constexpr int LIST_CAP = 512;
+// pending-path list: a power of two above the most it holds (RB - 1 left over + 2 RB new)
+__host__ __device__ constexpr int r32_list(int block) { return 4 * block; }
 
 __host__ __device__ inline size_t a16(size_t x) { return (x + 15) & ~size_t(15); }
 
@@ -66,7 +64,7 @@ struct R32Layout
     size_t slab, node, ir, bucket, listIdx, cnt, mbar, stepc, invn, rows, base, total;
 };
 
-__host__ __device__ inline R32Layout r32_layout(int rng, const McParams& p)
+__host__ __device__ inline R32Layout r32_layout(int rng, int block, const McParams& p)
 {
     R32Layout L;
     size_t off = 0;
@@ -78,10 +76,10 @@ __host__ __device__ inline R32Layout r32_layout(int rng, const McParams& p)
     off += a16(size_t(p.nS + 1) * 8);
     L.bucket = off;  // per bucket: its first knot's interval l0 and the knot above (xs[l0 + 1])
     off += a16(size_t(p.nBucketsF) * 8);
-    L.listIdx = off;  // (ring slot << 8) | (thread << 1) | path of the pair
-    off += a16(size_t(LIST_CAP) * 2);
-    L.cnt = off;    // per-warp counts, then the claimed chunk (first round, rounds)
-    off += 32;
+    L.listIdx = off;  // (ring slot * threads + thread) * 2 + path of the pair
+    off += a16(size_t(r32_list(block)) * 2);
+    L.cnt = off;    // the claimed chunk (first round, rounds), then per-warp counts
+    off += 16 + size_t(block / 32) * 4;
     L.mbar = off;   // completion barriers of the two row buffers
     off += 16;
     L.stepc = off;  // per-step node columns and weights of the reverse
@@ -91,30 +89,34 @@ __host__ __device__ inline R32Layout r32_layout(int rng, const McParams& p)
     L.rows = off;   // two buffers of rowChunk local-vol rows (y - 2d, d)[nS + 1]
     if (p.rowChunk) off += a16(size_t(2) * p.rowChunk * (p.nS + 1) * 8);
     L.base = off;
-    if (rng == RNG_SOBOL) off += a16(size_t(RW) * (size_t(p.nSteps) | 1) * 4);
+    if (rng == RNG_SOBOL) off += a16(size_t(block / 32) * (size_t(p.nSteps) | 1) * 4);
     L.total = off;
     return L;
 }
 
 // Nine blocks per SM (56 registers) where that costs no spills: the kernel is bound by issue
 // and latency, and a ninth block hides more of it (60x30 barrier, mrg32k3a: 3.8% faster).  The
-// Sobol barrier variant would spill at 56 registers and keeps eight.
-template <int PROD, int RNGK, bool ROWS>
-__global__ void __launch_bounds__(RB, (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 8 : 9)
+// Sobol barrier variant would spill at 56 registers and keeps eight.  Where shared memory holds fewer
+// blocks (the node slab and the step table of a 120x60 grid with 520 steps leave five), blocks of
+// 256 threads share them: four of those fit, 1024 threads per SM for 640 (200001 paths of that
+// barrier's risk: 1.16 -> 0.86 ms).
+template <int PROD, int RNGK, bool ROWS, int RB>
+__global__ void __launch_bounds__(RB, RB > 128 ? 4 : (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 8 : 9)
     dupire_risk32(const McParams p)
 {
     constexpr int NP = RNGK == RNG_MRG ? 2 : 1;
     constexpr bool UOC = PROD == PROD_UOC;
+    constexpr int RW = RB / 32, LIST_CAP = r32_list(RB);
     extern __shared__ __align__(128) unsigned char smem[];
-    const R32Layout L = r32_layout(RNGK, p);
+    const R32Layout L = r32_layout(RNGK, RB, p);
     long long* slab = reinterpret_cast<long long*>(smem + L.slab);  // [0,2) spot adjoint, payoffs from 8
     long long* paySlab = slab + 8;
     int* node = reinterpret_cast<int*>(smem + L.node);
     float2* sIr = reinterpret_cast<float2*>(smem + L.ir);
     int2* sBucket = reinterpret_cast<int2*>(smem + L.bucket);
     unsigned short* listIdx = reinterpret_cast<unsigned short*>(smem + L.listIdx);
-    int* cnt = reinterpret_cast<int*>(smem + L.cnt);
-    long long* sClaim = reinterpret_cast<long long*>(smem + L.cnt + 16);
+    long long* sClaim = reinterpret_cast<long long*>(smem + L.cnt);
+    int* cnt = reinterpret_cast<int*>(smem + L.cnt + 16);
     unsigned long long* mbar = reinterpret_cast<unsigned long long*>(smem + L.mbar);
     int4* sStepc = reinterpret_cast<int4*>(smem + L.stepc);
     float4* sInvn = reinterpret_cast<float4*>(smem + L.invn);
@@ -426,10 +428,10 @@ __global__ void __launch_bounds__(RB, (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 
         }
         const unsigned lt = (1u << lane) - 1u;
         if (live[0])
-            listIdx[(off + __popc(b0 & lt)) & (LIST_CAP - 1)] = (unsigned short)((slot << 8) | (tid << 1));
+            listIdx[(off + __popc(b0 & lt)) & (LIST_CAP - 1)] = (unsigned short)(slot * (2 * RB) + (tid << 1));
         if (NP == 2 && live[NP - 1])
             listIdx[(off + __popc(b0) + __popc(b1 & lt)) & (LIST_CAP - 1)] =
-                (unsigned short)((slot << 8) | (tid << 1) | 1);
+                (unsigned short)(slot * (2 * RB) + (tid << 1) + 1);
         __syncthreads();
         return total;
     };
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(RB, (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 
             const int e = listIdx[(head + tid) & (LIST_CAP - 1)];
             const int a = e & 1;
             const int col = int(blockIdx.x) * RB + ((e >> 1) & (RB - 1));
-            const float* es = scr + (e >> 8) * slotStride;  // the path's ring slot
+            const float* es = scr + e / (2 * RB) * slotStride;  // the path's ring slot
             float ax = es[(F_W + a) * rowStride + seedRow + col];
             float aAl = UOC ? es[(F_B + a) * rowStride + seedRow + col] : 0.0f;
             const unsigned* sw = reinterpret_cast<const unsigned*>(es) + (F_W + a) * rowStride + col;
@@ -676,14 +678,20 @@ __global__ void __launch_bounds__(RB, (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 
 
 }  // namespace
 
-template <bool ROWS>
-const void* dupire_risk32_ptr_t(int prod, int rng)
+template <bool ROWS, int RB>
+const void* dupire_risk32_ptr_b(int prod, int rng)
 {
-    if (prod == PROD_UOC && rng == RNG_MRG) return (const void*)&dupire_risk32<PROD_UOC, RNG_MRG, ROWS>;
-    if (prod == PROD_UOC && rng == RNG_SOBOL) return (const void*)&dupire_risk32<PROD_UOC, RNG_SOBOL, ROWS>;
-    if (prod == PROD_EUROPEAN && rng == RNG_MRG) return (const void*)&dupire_risk32<PROD_EUROPEAN, RNG_MRG, ROWS>;
-    if (prod == PROD_EUROPEAN && rng == RNG_SOBOL) return (const void*)&dupire_risk32<PROD_EUROPEAN, RNG_SOBOL, ROWS>;
+    if (prod == PROD_UOC && rng == RNG_MRG) return (const void*)&dupire_risk32<PROD_UOC, RNG_MRG, ROWS, RB>;
+    if (prod == PROD_UOC && rng == RNG_SOBOL) return (const void*)&dupire_risk32<PROD_UOC, RNG_SOBOL, ROWS, RB>;
+    if (prod == PROD_EUROPEAN && rng == RNG_MRG) return (const void*)&dupire_risk32<PROD_EUROPEAN, RNG_MRG, ROWS, RB>;
+    if (prod == PROD_EUROPEAN && rng == RNG_SOBOL) return (const void*)&dupire_risk32<PROD_EUROPEAN, RNG_SOBOL, ROWS, RB>;
     return nullptr;
+}
+
+template <bool ROWS>
+const void* dupire_risk32_ptr_t(int prod, int rng, int block)
+{
+    return block == 256 ? dupire_risk32_ptr_b<ROWS, 256>(prod, rng) : dupire_risk32_ptr_b<ROWS, 128>(prod, rng);
 }
 
 }  // namespace cf

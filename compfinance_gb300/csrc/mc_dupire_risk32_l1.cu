@@ -4,8 +4,8 @@
 
 namespace cf {
 
-const void* dupire_risk32_ptr_l1(int prod, int rng) { return dupire_risk32_ptr_t<false>(prod, rng); }
+const void* dupire_risk32_ptr_l1(int prod, int rng, int block) { return dupire_risk32_ptr_t<false>(prod, rng, block); }
 
-size_t dupire_risk32_smem(int rng, const McParams& p) { return r32_layout(rng, p).total; }
+size_t dupire_risk32_smem(int rng, int block, const McParams& p) { return r32_layout(rng, block, p).total; }
 
 }  // namespace cf

@@ -4,6 +4,6 @@
 
 namespace cf {
 
-const void* dupire_risk32_ptr_tma(int prod, int rng) { return dupire_risk32_ptr_t<true>(prod, rng); }
+const void* dupire_risk32_ptr_tma(int prod, int rng, int block) { return dupire_risk32_ptr_t<true>(prod, rng, block); }
 
 }  // namespace cf

@@ -13,19 +13,23 @@ const void* mc_kernel_ptr_bs_f64(int prod, int rng, int risk);
 const void* mc_kernel_ptr_bs_f32(int prod, int rng, int risk);
 const void* mc_kernel_ptr_dupire_f64(int prod, int rng, int risk);
 const void* mc_kernel_ptr_dupire_f32(int prod, int rng, int risk);
-const void* dupire_risk32_ptr_l1(int prod, int rng);
-const void* dupire_risk32_ptr_tma(int prod, int rng);
-size_t dupire_risk32_smem(int rng, const McParams& p);
+const void* dupire_risk32_ptr_l1(int prod, int rng, int block);
+const void* dupire_risk32_ptr_tma(int prod, int rng, int block);
+size_t dupire_risk32_smem(int rng, int block, const McParams& p);
 const void* dupire_fx64_ptr_european(int rng, int risk, int block);
 const void* dupire_fx64_ptr_uoc(int rng, int risk, int block);
 size_t dupire_fx64_smem(int rng, int block, const McParams& p);
+
+static int threads_of(const McLaunch& l) { return l.fast && l.block ? l.block : MC_BLOCK; }
 
 static const void* kernel_ptr(const McLaunch& l)
 {
     if (l.fast == 3)
         return l.prod == PROD_UOC ? dupire_fx64_ptr_uoc(l.rng, l.risk, l.block)
                                   : dupire_fx64_ptr_european(l.rng, l.risk, l.block);
-    if (l.fast) return l.fast == 2 ? dupire_risk32_ptr_tma(l.prod, l.rng) : dupire_risk32_ptr_l1(l.prod, l.rng);
+    if (l.fast)
+        return l.fast == 2 ? dupire_risk32_ptr_tma(l.prod, l.rng, threads_of(l))
+                           : dupire_risk32_ptr_l1(l.prod, l.rng, threads_of(l));
     if (l.model == MODEL_BS)
         return l.fp32 ? mc_kernel_ptr_bs_f32(l.prod, l.rng, l.risk) : mc_kernel_ptr_bs_f64(l.prod, l.rng, l.risk);
     return l.fp32 ? mc_kernel_ptr_dupire_f32(l.prod, l.rng, l.risk)
@@ -39,7 +43,7 @@ int mc_smem_bytes(const McLaunch& l, const McParams& p, int stageY, size_t* byte
         *bytes = dupire_fx64_smem(l.rng, l.block, p);
         return 0;
     }
-    *bytes = l.fast ? dupire_risk32_smem(l.rng, p) : mc_layout(l.model, l.rng, l.fp32, stageY, p, MC_BLOCK).total;
+    *bytes = l.fast ? dupire_risk32_smem(l.rng, threads_of(l), p) : mc_layout(l.model, l.rng, l.fp32, stageY, p, MC_BLOCK).total;
     return 0;
 }
 
@@ -70,7 +74,7 @@ int mc_scratch_fields(const McLaunch& l, long long rounds)
 
 size_t mc_scratch_bytes(const McLaunch& l, McParams& p, long long grid)
 {
-    const size_t fields = size_t(p.scratchFields) * size_t(p.nSteps + 1) * size_t(grid) * (l.fast == 3 ? l.block : MC_BLOCK) * (l.fp32 ? 4 : 8);
+    const size_t fields = size_t(p.scratchFields) * size_t(p.nSteps + 1) * size_t(grid) * threads_of(l) * (l.fp32 ? 4 : 8);
     if (!l.fast || l.fast == 3)
     {
         p.nodeSlabOffset = 0;
@@ -85,6 +89,23 @@ int mc_use_fast32(const McParams& plan, int prod, int fp32, int risk)
     if (!plan.fast32 || !fp32 || !risk || (prod != PROD_UOC && prod != PROD_EUROPEAN)) return 0;
     const char* env = std::getenv("CF_FAST32");
     return env && env[0] == '0' ? 0 : 1;
+}
+
+int r32_block(McLaunch& l, McParams& p, long long threadsNeeded, int numSMs)
+{
+    l.block = 128;
+    size_t b = 0;
+    int o1 = 0, o2 = 0;
+    p.stageY = p.rowChunk = 0;
+    mc_smem_bytes(l, p, 0, &b);
+    if (b > 200 * 1024 || mc_occupancy(l, b, &o1) || o1 < 1) return 0;
+    if (threadsNeeded > (long long)numSMs * o1 * 128)
+    {
+        l.block = 256;
+        mc_smem_bytes(l, p, 0, &b);
+        if (b > 200 * 1024 || mc_occupancy(l, b, &o2) || o2 * 256 <= o1 * 128) l.block = 128;
+    }
+    return l.block == 256 ? o2 : o1;
 }
 
 int r32_staging(McLaunch& l, McParams& p, int occ0, size_t* smem)
@@ -141,8 +162,7 @@ int mc_occupancy(const McLaunch& l, size_t smem, int* blocksPerSM)
     if (!fn) return (int)cudaErrorInvalidDeviceFunction;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, fn, l.fast == 3 ? l.block : MC_BLOCK,
-                                                              smem);
+    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, fn, threads_of(l), smem);
 }
 
 int launch_mc(const McLaunch& l, const McParams& p, void* stream)
@@ -151,7 +171,7 @@ int launch_mc(const McLaunch& l, const McParams& p, void* stream)
     if (!fn) return (int)cudaErrorInvalidDeviceFunction;
     McParams q = p;
     void* args[] = {&q};
-    return (int)cudaLaunchKernel(fn, dim3(l.grid), dim3(l.fast == 3 ? l.block : MC_BLOCK), args, l.smem, (cudaStream_t)stream);
+    return (int)cudaLaunchKernel(fn, dim3(l.grid), dim3(threads_of(l)), args, l.smem, (cudaStream_t)stream);
 }
 
 }  // namespace cf

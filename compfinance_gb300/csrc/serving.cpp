@@ -298,7 +298,7 @@ int cf_server_submit(cf_server* s, const cf_request* r, uint64_t* id)
     size_t fp = s->ctx->c.footprint(*plan, r->num, r->kind != 0);
     if (fp > s->sched.budget() && r->kind != 0)
     {
-        // an FP64 risk whose fixed-point form's scratch exceeds the budget runs the generic kernel
+        // a risk whose scratch exceeds the budget runs its smaller form
         const size_t small = s->ctx->c.footprint(*plan, r->num, true, true);
         q.generic = small < fp;
         fp = std::min(fp, small);

@@ -6,24 +6,37 @@
 
 namespace cf {
 
-// v 2^sft, rounded, into word i: the low two 32-bit adds return their old values for the carries; the
-// third is rarely needed (a negative value's sign word nearly always meets a carry).
-__device__ __forceinline__ void fx_node_add(unsigned* node, int nNodes, int i, long long v, int sft)
+// v[k] 2^sft, rounded, into words at[k], k < n (2 or 4).  Of each word the low two 32-bit adds return
+// their old values for the carries; the third is rarely needed (a negative value's sign word nearly
+// always meets a carry).  The adds of one kind are issued together: one after the other, each with
+// its carry, four words cost eight round trips to shared memory instead of two.
+__device__ __forceinline__ void fx_node_add(unsigned* node, int nNodes, const int (&at)[4], long long (&v)[4], int n, int sft)
 {
+    unsigned a1[4], a2[4], o[4];
     if (sft < 0)
     {
-        v = sft < -62 ? 0 : (v + (1LL << (-sft - 1))) >> -sft;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = sft < -62 ? 0 : (v[k] + (1LL << (-sft - 1))) >> -sft;
         sft = 0;
     }
-    const unsigned l = (unsigned)v, h = (unsigned)((unsigned long long)v >> 32);
-    const unsigned a0 = l << sft, a1 = __funnelshift_l(l, h, sft);
-    unsigned a2 = (unsigned)((int)h >> (sft ? 32 - sft : 31));
-    unsigned* at = node + i;
-    const unsigned o0 = atomicAdd(at, a0), c0 = o0 + a0 < o0 ? 1u : 0u;
-    const unsigned o1 = atomicAdd(at + nNodes, a1 + c0);
-    // a1 + c0 wraps to 0 only with a carry of its own
-    a2 += (a1 + c0 < c0 ? 1u : 0u) + (o1 + (a1 + c0) < o1 ? 1u : 0u);
-    if (a2) atomicAdd(at + 2 * nNodes, a2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (k < 2 || n > 2) o[k] = atomicAdd(node + at[k], (unsigned)v[k] << sft);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+        const unsigned l = (unsigned)v[k], h = (unsigned)((unsigned long long)v[k] >> 32), a0 = l << sft;
+        const unsigned c = o[k] + a0 < o[k] ? 1u : 0u, b1 = __funnelshift_l(l, h, sft);
+        a1[k] = b1 + c;
+        a2[k] = (unsigned)((int)h >> (sft ? 32 - sft : 31)) + (a1[k] < c ? 1u : 0u);  // b1 + c may wrap to 0
+        if (k < 2 || n > 2) o[k] = atomicAdd(node + nNodes + at[k], a1[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+        a2[k] += o[k] + a1[k] < o[k] ? 1u : 0u;
+        if (a2[k] && (k < 2 || n > 2)) atomicAdd(node + 2 * nNodes + at[k], a2[k]);
+    }
 }
 
 // Adjoint av of the vol sqrt(dt) sigma of step s at state y in interval lo, split over the interval's
@@ -52,14 +65,9 @@ __device__ __forceinline__ void fx_vol_adjoint(const McParams& p, long long* acc
         const long long N = hi < 0 ? -(long long)m : (long long)m;
         const long long nR = fx_mul_add(N * 32, t, 0), nL = N - nR;
         const long long rB = fx_mul_add(nR * 4, s0.x, 0), lB = fx_mul_add(nL * 4, s0.x, 0);
-        const int at = jl * nT;
-        fx_node_add(node, nNodes, at + col.x, nL - lB, sft);
-        fx_node_add(node, nNodes, at + col.y, lB, sft);
-        if (inner)
-        {
-            fx_node_add(node, nNodes, at + nT + col.x, nR - rB, sft);
-            fx_node_add(node, nNodes, at + nT + col.y, rB, sft);
-        }
+        const int at[4] = {jl * nT + col.x, jl * nT + col.y, (jl + 1) * nT + col.x, (jl + 1) * nT + col.y};
+        long long v[4] = {nL - lB, lB, nR - rB, rB};
+        fx_node_add(node, nNodes, at, v, inner ? 4 : 2, sft);
     }
     else
     {
@@ -87,8 +95,9 @@ __device__ __forceinline__ void fx_node_flush(long long* acc, unsigned* node, in
             node[i] = node[i + nNodes] = node[i + 2 * nNodes] = 0;
             const long long lo = (long long)(((unsigned long long)(n1 & 0xffu) << 32) | n0);  // 40 bits
             const long long hi = (long long)(((unsigned long long)n2 << 32) | n1) >> 8;
-            if (hi) atomicAdd(reinterpret_cast<unsigned long long*>(&acc[2 * (1 + i)]), (unsigned long long)hi);
-            if (lo) atomicAdd(reinterpret_cast<unsigned long long*>(&acc[2 * (1 + i) + 1]), (unsigned long long)lo);
+            long long* at = acc + 2 * (1 + i);
+            if (hi) atomicAdd(reinterpret_cast<unsigned long long*>(at), (unsigned long long)hi);
+            if (lo) atomicAdd(reinterpret_cast<unsigned long long*>(at + 1), (unsigned long long)lo);
         }
     }
 }

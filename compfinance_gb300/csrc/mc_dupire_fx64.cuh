@@ -269,28 +269,46 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
             double ax = __longlong_as_double(ey[seedRow]);
             double aAl = UOC ? __longlong_as_double(eb[seedRow]) : 0.0;
             ax *= 0x1p-59;  // carried in the Gaussians' unit
-            // states and Gaussians are loaded two steps ahead
-            long long yA = __ldcs(ey + (nSteps - 1) * Ti), gA = __ldcs(es + (nSteps - 1) * Ti), yB = 0, gB = 0;
+            // states and Gaussians are loaded three steps ahead (they come from DRAM), the vol and the slope of
+            // a step one step ahead of its adds
+            long long yA = __ldcs(ey + (nSteps - 1) * Ti), gA = __ldcs(es + (nSteps - 1) * Ti), yB = 0, gB = 0, yC = 0, gC = 0;
             if (nSteps >= 2)
             {
                 yB = __ldcs(ey + (nSteps - 2) * Ti);
                 gB = __ldcs(es + (nSteps - 2) * Ti);
             }
+            if (nSteps >= 3)
+            {
+                yC = __ldcs(ey + (nSteps - 3) * Ti);
+                gC = __ldcs(es + (nSteps - 3) * Ti);
+            }
+            int lo = fx_interval(sBucket, nBuckets, bShift, x0h, yA);
+            int4 vc = __ldg(reinterpret_cast<const int4*>(vols + (nSteps - 1) * pitch + lo));
+            double slope = __ldg(p.fx.slope + (nSteps - 1) * pitch + lo);
             for (int s = nSteps - 1; s >= 0; --s)
             {
                 const long long y = yA, g = a ? -gA : gA;
+                const long long v = fx_vol((long long)(((unsigned long long)(unsigned)vc.y << 32) | (unsigned)vc.x), vc.z, vc.w,
+                                           y, center, dShift);
+                const double av = ax * (double)(g - 2 * (v >> (4 - r)));  // d y_{s+1} / d v = g - v
+                ax = fma(av, slope, ax);
+                const int k = lo;
                 yA = yB;
                 gA = gB;
-                if (s >= 2)
+                yB = yC;
+                gB = gC;
+                if (s >= 3)
                 {
-                    yB = __ldcs(ey + (s - 2) * Ti);
-                    gB = __ldcs(es + (s - 2) * Ti);
+                    yC = __ldcs(ey + (s - 3) * Ti);
+                    gC = __ldcs(es + (s - 3) * Ti);
                 }
-                int lo;
-                const long long v = volAt(s, y, lo);
-                const double av = ax * (double)(g - 2 * (v >> (4 - r)));  // d y_{s+1} / d v = g - v
-                ax = fma(av, __ldg(p.fx.slope + s * pitch + lo), ax);
-                if (av != 0.0) fx_vol_adjoint(p, p.acc, node, nNodes, sIv, sInv, s, lo, y, av);
+                if (s >= 1)
+                {
+                    lo = fx_interval(sBucket, nBuckets, bShift, x0h, yA);
+                    vc = __ldg(reinterpret_cast<const int4*>(vols + (s - 1) * pitch + lo));
+                    slope = __ldg(p.fx.slope + (s - 1) * pitch + lo);
+                }
+                if (av != 0.0) fx_vol_adjoint(p, p.acc, node, nNodes, sIv, sInv, s, k, y, av);
                 // the date at point s: survival below the barrier's smoothing band
                 if (UOC && y > yBand && aAl != 0.0 && (evEvery ? s > 0 || p.evAtStep[0] >= 0 : __ldg(p.evAtStep + s) >= 0))
                 {

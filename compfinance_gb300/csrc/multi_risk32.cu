@@ -411,8 +411,9 @@ __global__ void __launch_bounds__(MB) multi32_reverse(const Multi32Args A)
     {
         if (tid == 0) misc[0] = atomicAdd(A.work, 1);
         __syncthreads();
-        const int c = misc[0];
-        if (c >= nChunks) break;
+        // the last maturities, whose sweeps are the longest, first
+        const int c = nChunks - 1 - misc[0];
+        if (c < 0) break;
         // bucket of chunk c: the last b with chunkStart[b] <= c (empty buckets share starts)
         int lo = 0, hi = nB;
         while (hi - lo > 1)

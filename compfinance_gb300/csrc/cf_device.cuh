@@ -374,6 +374,14 @@ __device__ __forceinline__ unsigned sobol_state(const unsigned* dir, int stride,
     return s;
 }
 
+// State of index l in [0, 32): what a warp's lane XORs to the state of its batch's first index, from
+// the table [dimension][32] (one coalesced load; the loop over the set bits took a warp five rounds
+// of it at every draw).
+__device__ __forceinline__ unsigned sobol_low(const McParams& p, int d, int lane)
+{
+    return __ldg(p.sobolLow + d * 32 + lane);
+}
+
 // ---------------------------------------------------------------------------------------
 // Bulk copies global -> shared through the TMA unit (cp.async.bulk, no tensor map), with
 // completion tracked by an mbarrier.  Every wait is bounded.  A wait that expires records

@@ -120,7 +120,8 @@ struct McParams
 
     // random numbers
     unsigned seed1, seed2;
-    const unsigned* sobolDir;              // [32][nSteps]
+    const unsigned* sobolDir;              // [32][dimensions]
+    const unsigned* sobolLow;              // [dimensions][32] states of the indexes below 32
     const unsigned* mrgJumpA;  // jump tables of the first component (mrg_jump)
     const unsigned* mrgJumpB;  // and of the second
 

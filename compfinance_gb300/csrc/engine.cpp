@@ -665,17 +665,9 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
     std::vector<int> po = pd.payOff;
     if (po.empty()) po = {0, 0};
     const size_t oK = pk.vec(kf), oKf = pk.vec(to_f(kf)), oPo = pk.vec(po);
-    size_t oDir = 0;
-    if (plan.nSteps <= sobol_max_dim())
-    {
-        auto& dirs = sobolDirs[plan.nSteps];  // regenerated once per dimension count
-        if (dirs.empty()) dirs = sobol_dirs(plan.nSteps);
-        oDir = pk.vec(dirs);
-    }
     plan.sobolOk = plan.nSteps <= sobol_max_dim();
-
-    int rc = plan.tables.ensure(pk.buf.size());
-    if (rc) return rc;
+    int rc = plan.sobolOk ? sobolTables(plan.nSteps, P) : CF_OK;
+    if (rc || (rc = plan.tables.ensure(pk.buf.size()))) return rc;
     CF_CUDA(cudaMemcpyAsync(plan.tables.ptr, pk.buf.data(), pk.buf.size(), cudaMemcpyHostToDevice, stream));
     h2d += pk.buf.size();
     // the tables are read by kernels on any slot's stream: the upload completes here
@@ -720,7 +712,6 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
     P.kD = (const double*)D(oK);
     P.kF = (const float*)D(oKf);
     P.evPayOff = (const int*)D(oPo);
-    P.sobolDir = plan.sobolOk ? (const unsigned*)D(oDir) : nullptr;
     plan.evAtStep = evAtStep;
     P.evEvery = 1;
     for (int i = 1; i <= plan.nSteps; ++i)
@@ -772,6 +763,26 @@ Context::~Context()
     cudaSetDevice(device);
     plans.clear();
     if (ownStream) cudaStreamDestroy(ownStream);
+}
+
+int Context::sobolTables(int dim, McParams& p)
+{
+    DevBuf& b = sobolTabs[dim];
+    if (!b.ptr)
+    {
+        std::vector<uint32_t> t = sobol_dirs(dim);
+        t.resize(size_t(64) * dim, 0u);
+        uint32_t* low = t.data() + size_t(32) * dim;
+        for (int d = 0; d < dim; ++d)
+            for (int l = 1; l < 32; ++l) low[d * 32 + l] = low[d * 32 + l - 1] ^ t[size_t(__builtin_ctz(l)) * dim + d];
+        int rc = b.ensure(t.size() * 4);
+        if (rc) return rc;
+        CF_CUDA(cudaMemcpy(b.ptr, t.data(), t.size() * 4, cudaMemcpyHostToDevice));
+        h2d += t.size() * 4;
+    }
+    p.sobolDir = static_cast<const unsigned*>(b.ptr);
+    p.sobolLow = p.sobolDir + size_t(32) * dim;
+    return CF_OK;
 }
 
 int Context::getPlan(const std::string& mid, const std::string& pid, Plan*& out)

@@ -181,7 +181,10 @@ struct Context
     std::map<std::string, ProductDesc> products;
     std::map<std::pair<std::string, std::string>, std::shared_ptr<Plan>> plans;
     DevBuf jump;
-    std::map<int, std::vector<uint32_t>> sobolDirs;  // Sobol direction numbers per dimension count
+    // per dimension count: Sobol direction numbers [32][dim] and, after them, the states of the
+    // indexes below 32, [dim][32] (at most 1101 counts, 0.3 MB each)
+    std::map<int, DevBuf> sobolTabs;
+    int sobolTables(int dim, McParams& p);
     const unsigned* jumpA = nullptr;
     const unsigned* jumpB = nullptr;
     DevBuf invn;  // piecewise-cubic inverse normal tables of the FP32 kernels: mrg32k3a, Sobol

@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
                 }
                 const int slot = RISK ? slotOf(it) : 0;
                 forward(nAct, n - 1, [&](int i) {
-                    return sobol_gauss_fx(p.fx, base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
+                    return sobol_gauss_fx(p.fx, base[i] ^ sobol_low(p, i, lane));
                 });
                 if (RISK) endRound(slot);
             }

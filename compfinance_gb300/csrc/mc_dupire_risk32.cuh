@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(RB, RB > 128 ? 4 : (PROD == PROD_UOC && RNGK =
                 }
                 const int slot = slotOf(it);
                 if (!forward(nAct, [&](int i) {
-                        const unsigned sb = base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane);
+                        const unsigned sb = base[i] ^ sobol_low(p, i, lane);
                         const bool sup = sb >= 2147483648u;
                         return gaussT(sup ? 0u - sb : (sb > 1u ? sb : 1u), sup);  // state 0 occurs only at index 0
                     }))

@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
                 const int nAct = (n >= 1 && n <= p.nPath) ? 1 : 0;
                 if (ROWACC || nAct)
                     runUnit(nAct, n - 1, [&](int i) {
-                        return sobol_gauss<Real>(p.fx, base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
+                        return sobol_gauss<Real>(p.fx, base[i] ^ sobol_low(p, i, lane));
                     });
             }
         }

@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 ? 1 : sizeof(Real) == 4 ? (RN
             const long long n = b * 32 + lane;
             if (n >= 1 && n <= p.nPath)
                 runUnit(1, [&](int d) {
-                    return sobol_gauss<Real>(p.fx, base[d] ^ sobol_state(p.sobolDir, dim, d, (unsigned long long)lane));
+                    return sobol_gauss<Real>(p.fx, base[d] ^ sobol_low(p, d, lane));
                 });
         }
     }

@@ -268,14 +268,8 @@ int Context::buildPlanMd(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
     const size_t oDyn = put(dyn.data(), dyn.size() * 4), oEv = put(evAtStep.data(), evAtStep.size() * 4);
     const int dim = nS * nA;
     plan.sobolOk = dim <= sobol_max_dim();
-    size_t oDir = 0;
-    if (plan.sobolOk)
-    {
-        const std::vector<unsigned> dirs = sobol_dirs(dim);
-        oDir = put(dirs.data(), dirs.size() * 4);
-    }
-    int rc = plan.tables.ensure(buf.size());
-    if (rc) return rc;
+    int rc = plan.sobolOk ? sobolTables(dim, P) : CF_OK;
+    if (rc || (rc = plan.tables.ensure(buf.size()))) return rc;
     CF_CUDA(cudaMemcpyAsync(plan.tables.ptr, buf.data(), buf.size(), cudaMemcpyHostToDevice, stream));
     // the pageable source must outlive the copy
     CF_CUDA(cudaStreamSynchronize(stream));
@@ -289,7 +283,6 @@ int Context::buildPlanMd(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
     P.kF = reinterpret_cast<const float*>(dv + oKF);
     P.mdDyn = reinterpret_cast<const int*>(dv + oDyn);
     P.evAtStep = reinterpret_cast<const int*>(dv + oEv);
-    P.sobolDir = plan.sobolOk ? reinterpret_cast<const unsigned*>(dv + oDir) : nullptr;
     P.acKo = pd.ko;
     P.acStrike = pd.strike;
     P.acCpn = pd.cpn;

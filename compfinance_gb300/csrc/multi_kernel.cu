@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(MC_BLOCK) multi_kernel(const MultiParams mp)
             const long long n = b * 32 + lane;
             if (n >= 1 && n <= p.nPath)
                 runUnit(1, [&](int i) {
-                    return sobol_gauss<Real>(p.fx, base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
+                    return sobol_gauss<Real>(p.fx, base[i] ^ sobol_low(p, i, lane));
                 });
         }
     }

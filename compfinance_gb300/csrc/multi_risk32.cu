@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(MB) multi32_forward(const Multi32Args A)
             const long long n = b * 32 + lane;
             if (n >= 1 && n <= nPath)
                 runUnit(1, n - 1, [&](int i) {
-                    const unsigned sb = base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane);
+                    const unsigned sb = base[i] ^ sobol_low(p, i, lane);
                     const bool sup = sb >= 2147483648u;
                     return gaussT(sup ? 0u - sb : (sb > 1u ? sb : 1u), sup);
                 });

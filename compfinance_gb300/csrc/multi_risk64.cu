@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(FB, 8) multi64_forward(const Multi32Args A)
             const long long n = b * 32 + lane;
             if (n >= 1 && n <= nPath)
                 runUnit(1, n - 1, [&](int i) {
-                    return sobol_gauss_fx(p.fx, base[i] ^ sobol_state(p.sobolDir, nSteps, i, (unsigned long long)lane));
+                    return sobol_gauss_fx(p.fx, base[i] ^ sobol_low(p, i, lane));
                 });
         }
     }

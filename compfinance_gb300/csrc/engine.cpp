@@ -862,14 +862,18 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
         wf[k] = float(wd[k]);
     }
     char* wbase = static_cast<char*>(slot.work.ptr);
-    CF_CUDA(cudaMemcpyAsync(wbase, wd, size_t(plan.nPay) * 12, cudaMemcpyHostToDevice, st));
-    h2d += size_t(plan.nPay) * 12;
+    if (weights)
+    {
+        CF_CUDA(cudaMemcpyAsync(wbase, wd, size_t(plan.nPay) * 12, cudaMemcpyHostToDevice, st));
+        h2d += size_t(plan.nPay) * 12;
+    }
     p.w = reinterpret_cast<const double*>(wbase);
     p.wf = reinterpret_cast<const float*>(wbase + size_t(plan.nPay) * 8);
     p.acc = reinterpret_cast<long long*>(wbase + wBytes);
     p.err = reinterpret_cast<int*>(wbase + wBytes + accBytes);
     p.claim = reinterpret_cast<unsigned long long*>(wbase + wBytes + accBytes + 16);
-    CF_CUDA(cudaMemsetAsync(p.acc, 0, accBytes + 16 + claimBytes, st));
+    // without weights theirs are zeros, cleared with the accumulators: one operation less before the kernel
+    CF_CUDA(cudaMemsetAsync(weights ? static_cast<void*>(p.acc) : wbase, 0, (weights ? 0 : wBytes) + accBytes + 16 + claimBytes, st));
 
     McLaunch l{plan.model, plan.prod, sobol ? RNG_SOBOL : RNG_MRG, fp32 ? 1 : 0, risk ? 1 : 0, 0, 0, 0, 0};
     // FP32 Dupire risk runs dupire_risk32 when the plan has its tables and its node slab fits

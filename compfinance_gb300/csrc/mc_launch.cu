@@ -6,6 +6,7 @@
 #include <cstdlib>
 
 #include "mc_kernel.cuh"
+#include "occupancy.h"
 
 namespace cf {
 
@@ -148,8 +149,6 @@ int r32_staging(McLaunch& l, McParams& p, int occ0, size_t* smem)
             }
         }
     }
-    // the chosen configuration is measured last: that also leaves the kernel's dynamic
-    // shared-memory limit at the size it launches with
     const int occ = occOf(stage, chunk, smem);
     if (occ >= 1) return occ;
     occOf(0, 0, smem);
@@ -160,9 +159,7 @@ int mc_occupancy(const McLaunch& l, size_t smem, int* blocksPerSM)
 {
     const void* fn = kernel_ptr(l);
     if (!fn) return (int)cudaErrorInvalidDeviceFunction;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocksPerSM, fn, threads_of(l), smem);
+    return kernel_occupancy(fn, threads_of(l), smem, blocksPerSM);
 }
 
 int launch_mc(const McLaunch& l, const McParams& p, void* stream)

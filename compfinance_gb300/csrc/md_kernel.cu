@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "cf_device.cuh"
+#include "occupancy.h"
 
 namespace cf {
 
@@ -482,9 +483,7 @@ int md_scratch_fields(int rng, const McParams& p)
 int md_occupancy(int rng, int fp32, int nA, size_t smem, int* occ)
 {
     const void* fn = md_ptr(rng, fp32, nA);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, fn, MD_BLOCK, smem);
-    return (int)e;
+    return kernel_occupancy(fn, MD_BLOCK, smem, occ);
 }
 
 int launch_md(int rng, int fp32, int grid, size_t smem, const McParams& p, void* stream)

@@ -326,14 +326,17 @@ int Context::enqueueMd(Slot& slot, Plan& plan, const cf_num_param& num, bool ris
         wf[k] = float(wd[k]);
     }
     char* wbase = static_cast<char*>(slot.work.ptr);
-    CF_CUDA(cudaMemcpyAsync(wbase, wd, size_t(plan.nPay) * 12, cudaMemcpyHostToDevice, st));
-    h2d += size_t(plan.nPay) * 12;
+    if (weights)
+    {
+        CF_CUDA(cudaMemcpyAsync(wbase, wd, size_t(plan.nPay) * 12, cudaMemcpyHostToDevice, st));
+        h2d += size_t(plan.nPay) * 12;
+    }
     p.w = reinterpret_cast<const double*>(wbase);
     p.wf = reinterpret_cast<const float*>(wbase + size_t(plan.nPay) * 8);
     p.acc = reinterpret_cast<long long*>(wbase + wBytes);
     p.err = reinterpret_cast<int*>(wbase + wBytes + accBytes);
     p.claim = reinterpret_cast<unsigned long long*>(wbase + wBytes + accBytes + 8);  // zeroed with the flag
-    CF_CUDA(cudaMemsetAsync(p.acc, 0, accBytes + 16, st));
+    CF_CUDA(cudaMemsetAsync(weights ? static_cast<void*>(p.acc) : wbase, 0, (weights ? 0 : wBytes) + accBytes + 16, st));
 
     const size_t smem = md_smem_bytes(rng, fp32, p);
     int occ = 0;

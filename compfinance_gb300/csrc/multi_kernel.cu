@@ -16,6 +16,7 @@
 
 #include "cf_device.cuh"
 #include "mc_kernel.cuh"
+#include "occupancy.h"
 
 namespace cf {
 
@@ -346,9 +347,7 @@ static const void* multi_ptr(int model, int rng, int fp32)
 int multi_occupancy(int model, int rng, int fp32, size_t smem, int* occ)
 {
     const void* fn = multi_ptr(model, rng, fp32);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, fn, MC_BLOCK, smem);
+    return kernel_occupancy(fn, MC_BLOCK, smem, occ);
 }
 
 // Per-payoff risks from the bucket accumulators.  Bucket m of a maturity holds the adjoints of

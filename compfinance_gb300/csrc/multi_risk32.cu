@@ -28,6 +28,7 @@
 
 #include "cf_device.cuh"
 #include "multi32.h"
+#include "occupancy.h"
 
 namespace cf {
 
@@ -534,12 +535,8 @@ size_t m32_reverse_smem(const Multi32Args& a) { return rev_layout(a).total; }
 
 int m32_occupancy(int rng, size_t smemFwd, size_t smemRev, int* occFwd, int* occRev)
 {
-    cudaError_t e = cudaFuncSetAttribute(fwd_ptr(rng), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemFwd);
-    if (!e) e = cudaFuncSetAttribute((const void*)&multi32_reverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smemRev);
-    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occFwd, fwd_ptr(rng), MB, smemFwd);
-    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occRev, (const void*)&multi32_reverse, MB, smemRev);
-    return (int)e;
+    const int e = kernel_occupancy(fwd_ptr(rng), MB, smemFwd, occFwd);
+    return e ? e : kernel_occupancy((const void*)&multi32_reverse, MB, smemRev, occRev);
 }
 
 int launch_multi32_scan(const Multi32Args& a, void* stream)

@@ -12,6 +12,7 @@
 
 #include "fx_device.cuh"
 #include "multi32.h"
+#include "occupancy.h"
 
 namespace cf {
 
@@ -290,12 +291,8 @@ size_t m64_reverse_smem(const Multi32Args& a) { return rev64_layout(a).total; }
 
 int m64_occupancy(int rng, size_t smemFwd, size_t smemRev, int* occFwd, int* occRev)
 {
-    const void* rev = (const void*)&multi64_reverse;
-    cudaError_t e = cudaFuncSetAttribute(fwd_ptr(rng), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemFwd);
-    if (!e) e = cudaFuncSetAttribute(rev, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemRev);
-    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occFwd, fwd_ptr(rng), FB, smemFwd);
-    if (!e) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occRev, rev, M64_BLOCK, smemRev);
-    return (int)e;
+    const int e = kernel_occupancy(fwd_ptr(rng), FB, smemFwd, occFwd);
+    return e ? e : kernel_occupancy((const void*)&multi64_reverse, M64_BLOCK, smemRev, occRev);
 }
 
 int launch_multi64(int rng, int gridFwd, size_t smemFwd, int gridRev, size_t smemRev, const Multi32Args& a,

@@ -382,6 +382,20 @@ __device__ __forceinline__ unsigned sobol_low(const McParams& p, int d, int lane
     return __ldg(p.sobolLow + d * 32 + lane);
 }
 
+// End of a launch, whole block, after its last adds into the accumulators: the last block to get here
+// writes the accumulators and the error flag to pinned host memory (a copy engine operation after
+// the kernel took 5 us more).
+__device__ __forceinline__ void results_out(const McParams& p)
+{
+    if (!p.hostOut) return;
+    __threadfence();
+    __syncthreads();
+    if (!__syncthreads_or(threadIdx.x == 0 && atomicAdd(p.err + 1, 1) == int(gridDim.x) - 1)) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < 2 * p.nAcc; i += blockDim.x) p.hostOut[i] = __ldcg(p.acc + i);
+    if (threadIdx.x == 0) p.hostOut[2 * p.nAcc] = (long long)*reinterpret_cast<volatile int*>(p.err);
+}
+
 // ---------------------------------------------------------------------------------------
 // Bulk copies global -> shared through the TMA unit (cp.async.bulk, no tensor map), with
 // completion tracked by an mbarrier.  Every wait is bounded.  A wait that expires records

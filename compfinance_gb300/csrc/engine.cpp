@@ -984,6 +984,7 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
         if (rc) return rc;
         p.scratch = slot.scratch.ptr;
     }
+    const bool handOver = p.nAcc <= HOST_OUT_MAX && (!l.fast || l.fast == 3);
     int nLaunch = 0;
     for (long long off = 0; off < totalPaths; off += chunk)
     {
@@ -991,13 +992,19 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
         q.firstPath = firstPath + off;
         q.nPath = std::min(chunk, totalPaths - off);
         q.claim = p.claim + nLaunch;
+        if (handOver && off + chunk >= totalPaths)  // the run's last launch
+        {
+            q.hostOut = static_cast<long long*>(slot.hostAcc.ptr);
+            q.hostOut[2 * size_t(p.nAcc)] = DEVERR_NO_RESULT;
+        }
         rc = launch_mc(l, q, st);
         if (rc) return cuda_fail(cudaError_t(rc), "mc_kernel launch");
         ++nLaunch;
     }
     p.nPath = totalPaths;  // the averages are over the whole run
-    CF_CUDA(cudaMemcpyAsync(slot.hostAcc.ptr, p.acc, accBytes + 16, cudaMemcpyDeviceToHost, st));
-    d2h += accBytes + 16;
+    if (!handOver)
+        CF_CUDA(cudaMemcpyAsync(slot.hostAcc.ptr, p.acc, accBytes + 8, cudaMemcpyDeviceToHost, st));
+    d2h += accBytes + 8;
     if (!slot.done) CF_CUDA(cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming));
     CF_CUDA(cudaEventRecord(slot.done, st));
     slot.last = p;

@@ -423,6 +423,7 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
     __syncthreads();
     if (RISK && tid == 0) fix_flush(&p.acc[0], &slab[0]);
     for (int i = tid; i < 2 * nPay + (RISK ? 2 : 0); i += RB) fix_flush(&p.acc[2 * (p.nRisk + i)], &paySlab[2 * i]);
+    results_out(p);
 }
 
 }  // namespace

@@ -712,6 +712,7 @@ __global__ void __launch_bounds__(MC_BLOCK) mc_kernel(const McParams p)
         }
     }
     for (int i = tid; i < 2 * nPay + 2; i += MC_BLOCK) fix_flush(&p.acc[2 * (p.nRisk + i)], &paySlab[2 * i]);
+    results_out(p);
 }
 
 }  // namespace cf

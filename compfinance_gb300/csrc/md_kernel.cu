@@ -453,6 +453,7 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 ? 1 : sizeof(Real) == 4 ? (RN
     }
     __syncthreads();
     for (int i = tid; i < p.nAcc; i += MD_BLOCK) fix_flush(&p.acc[2 * i], &sAcc[2 * i]);
+    results_out(p);
 }
 
 template <int RNGK, class Real>

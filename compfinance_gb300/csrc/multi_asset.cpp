@@ -351,10 +351,15 @@ int Context::enqueueMd(Slot& slot, Plan& plan, const cf_num_param& num, bool ris
         if ((rc = slot.scratch.ensure(fields * size_t(grid) * 128 * (fp32 ? 4 : 8), st))) return rc;
         p.scratch = slot.scratch.ptr;
     }
+    if (p.nAcc <= HOST_OUT_MAX)
+    {
+        p.hostOut = static_cast<long long*>(slot.hostAcc.ptr);  // written by the launch's last block
+        p.hostOut[2 * size_t(p.nAcc)] = DEVERR_NO_RESULT;
+    }
     rc = launch_md(rng, fp32, int(grid), smem, p, st);
     if (rc) return cuda_fail(cudaError_t(rc), "multi-asset kernel launch");
-    CF_CUDA(cudaMemcpyAsync(slot.hostAcc.ptr, p.acc, accBytes + 16, cudaMemcpyDeviceToHost, st));
-    d2h += accBytes + 16;
+    if (!p.hostOut) CF_CUDA(cudaMemcpyAsync(slot.hostAcc.ptr, p.acc, accBytes + 8, cudaMemcpyDeviceToHost, st));
+    d2h += accBytes + 8;
     if (!slot.done) CF_CUDA(cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming));
     CF_CUDA(cudaEventRecord(slot.done, st));
     slot.last = p;

@@ -103,6 +103,7 @@ struct FxParams
     const FxVol* vol;            // [nSteps][nS + 1]
     const double* slope;         // [nSteps][nS + 1] d vol / d y 2^-59
     const FxStep* step;          // [nSteps]
+    NodeStride node;             // of the reverse's slab
     // barrier smoothing band: y above yTop knocks out, above yBand survives by a factor linear in the
     // spot; bandScale > 0: the factor is bandScale times fx_one_minus_exp8(yTop - y)
     long long yTop, yBand;
@@ -223,7 +224,7 @@ struct McParams
     int nodeShiftF;
     long long nodeSlabOffset;
     const float* invnF;   // [512][4] piecewise-cubic inverse normal of the launch's generator
-    // dupire_risk32: per step (colA, colB, time weights A and B in units of 2^-nodeShiftF as
+    // dupire_risk32: per step (nS colA, nS colB, time weights A and B in units of 2^-nodeShiftF as
     // float bits), the node columns and weights of the reverse sweep's local-vol adjoints
     const int4* stepcF;
     // dupire_risk32: local-vol rows staged into shared memory by bulk copies, rowChunk steps per

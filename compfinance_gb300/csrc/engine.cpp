@@ -587,8 +587,8 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
             for (int i = 0; i < n; ++i)
             {
                 const float wa = std::ldexp(float(cAv[i]), P.nodeShiftF), wb = std::ldexp(float(cBv[i]), P.nodeShiftF);
-                scv[4 * size_t(i)] = colA[i];
-                scv[4 * size_t(i) + 1] = colB[i];
+                scv[4 * size_t(i)] = colA[i] * nS;  // the slab is held by time column
+                scv[4 * size_t(i) + 1] = colB[i] * nS;
                 std::memcpy(&scv[4 * size_t(i) + 2], &wa, 4);
                 std::memcpy(&scv[4 * size_t(i) + 3], &wb, 4);
             }
@@ -622,6 +622,7 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
             plan.fxTouch = sMax;
             in.sq = std::move(sqv);
             in.tw = std::move(twv);
+            in.node = pd.kind == PROD_EUROPEANS ? node_stride(nS, nT) : NodeStride{nT, 1};
             in.colA = std::move(colA);
             in.colB = std::move(colB);
         }
@@ -886,7 +887,7 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
     // threads for one unit each of n paths
     auto needOf = [sobol](long long n) { return sobol ? (n / 32 + 1) * 32 : (n + 1) / 2; };
     // FP64 Dupire European and barrier runs in fixed point at every size their tables fit: 60x30 weekly
-    // barrier risk 9.5 -> 0.62 ms at 2^18 paths (141 -> 5.6 ms at 2^22), its value 5.2 -> 0.30 ms,
+    // barrier risk 9.5 -> 0.59 ms at 2^18 paths (141 -> 5.6 ms at 2^22), its value 5.2 -> 0.30 ms,
     // 20x10 grid and 10^5 x 52 steps 0.85 -> 0.14 ms against the generic kernel
     if (!fp32 && !generic && plan.prod != PROD_EUROPEANS && fxReady(plan))
     {

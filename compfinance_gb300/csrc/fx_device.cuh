@@ -1,6 +1,6 @@
 // Reverse step of the fixed-point Dupire kernels (mc_dupire_fx64.cuh, multi_risk64.cu): the adjoint of
 // one step's vol into a slab of 96-bit words of the local-vol nodes in shared memory, in units of
-// 2^-60, held as three arrays of 32-bit words [3][nNodes].
+// 2^-60, held as three arrays of 32-bit words [3][nNodes], each laid out by node_stride().
 #pragma once
 #include "cf_device.cuh"
 
@@ -46,14 +46,14 @@ __device__ __forceinline__ void fx_vol_adjoint(const McParams& p, long long* acc
                                                const FxInterval* sIv, const long long* sInv, int s, int lo, long long y,
                                                double av)
 {
-    const int nS = p.nS, nT = p.nT;
+    const int nS = p.nS, dl = p.fx.node.l;
     const FxInterval iv = sIv[lo];
     const bool inner = lo > 0 && lo < nS;  // two knots; one at the flat ends
     // weight of the upper knot, units of 2^-59
     const long long t = inner ? fx_mul_add(sInv[lo], (long long)((unsigned long long)(y - iv.x) << iv.sh), 0) : 0;
     const int jl = lo - (lo > 0 ? 1 : 0);
     const longlong2 s0 = __ldg(reinterpret_cast<const longlong2*>(p.fx.step + s));
-    const int2 col = __ldg(reinterpret_cast<const int2*>(&p.fx.step[s].colA));
+    const int2 at2 = __ldg(reinterpret_cast<const int2*>(&p.fx.step[s].atA));
     // the adjoint of sigma as N 2^sft units of 2^-60: its 53-bit mantissa
     const double c = av * __longlong_as_double(s0.y);
     const int hi = __double2hiint(c), E = (hi >> 20) & 0x7ff;
@@ -65,7 +65,7 @@ __device__ __forceinline__ void fx_vol_adjoint(const McParams& p, long long* acc
         const long long N = hi < 0 ? -(long long)m : (long long)m;
         const long long nR = fx_mul_add(N * 32, t, 0), nL = N - nR;
         const long long rB = fx_mul_add(nR * 4, s0.x, 0), lB = fx_mul_add(nL * 4, s0.x, 0);
-        const int at[4] = {jl * nT + col.x, jl * nT + col.y, (jl + 1) * nT + col.x, (jl + 1) * nT + col.y};
+        const int at[4] = {jl * dl + at2.x, jl * dl + at2.y, (jl + 1) * dl + at2.x, (jl + 1) * dl + at2.y};
         long long v[4] = {nL - lB, lB, nR - rB, rB};
         fx_node_add(node, nNodes, at, v, inner ? 4 : 2, sft);
     }
@@ -73,6 +73,8 @@ __device__ __forceinline__ void fx_vol_adjoint(const McParams& p, long long* acc
     {
         const double cR = c * ((double)t * 0x1p-59), cL = c - cR;
         const double tw = (double)s0.x * 0x1p-62;
+        const int nT = p.nT;
+        const int2 col = __ldg(reinterpret_cast<const int2*>(&p.fx.step[s].colA));
         acc += 2 * (1 + jl * nT);
         fix_add(acc + 2 * col.x, cL - cL * tw);
         fix_add(acc + 2 * col.y, cL * tw);
@@ -85,21 +87,29 @@ __device__ __forceinline__ void fx_vol_adjoint(const McParams& p, long long* acc
 }
 
 // Whole block (threads of them): the slab into the accumulator pairs acc[1 + node], and cleared.
-__device__ __forceinline__ void fx_node_flush(long long* acc, unsigned* node, int nNodes, int threads)
+// STRIDED: the slab may be by time column (p.fx.node); without it the loop is by row alone, whose
+// second copy made a barrier's sweep 2% slower.
+template <bool STRIDED>
+__device__ __forceinline__ void fx_node_flush(const McParams& p, long long* acc, unsigned* node, int nNodes, int threads)
 {
-    for (int i = threadIdx.x; i < nNodes; i += threads)
-    {
-        const unsigned n0 = node[i], n1 = node[i + nNodes], n2 = node[i + 2 * nNodes];
+    const int nS = p.nS, nT = p.nT;
+    auto flush = [&](int i, int k) {
+        const unsigned n0 = node[k], n1 = node[k + nNodes], n2 = node[k + 2 * nNodes];
         if (n0 | n1 | n2)
         {
-            node[i] = node[i + nNodes] = node[i + 2 * nNodes] = 0;
+            node[k] = node[k + nNodes] = node[k + 2 * nNodes] = 0;
             const long long lo = (long long)(((unsigned long long)(n1 & 0xffu) << 32) | n0);  // 40 bits
             const long long hi = (long long)(((unsigned long long)n2 << 32) | n1) >> 8;
             long long* at = acc + 2 * (1 + i);
             if (hi) atomicAdd(reinterpret_cast<unsigned long long*>(at), (unsigned long long)hi);
             if (lo) atomicAdd(reinterpret_cast<unsigned long long*>(at + 1), (unsigned long long)lo);
         }
-    }
+    };
+    if (!STRIDED || p.fx.node.c == 1)
+        for (int i = threadIdx.x; i < nS * nT; i += threads) flush(i, i);
+    else
+        for (int l = threadIdx.x >> 5; l < nS; l += threads >> 5)
+            for (int c = threadIdx.x & 31; c < nT; c += 32) flush(l * nT + c, l * p.fx.node.l + c * p.fx.node.c);
 }
 
 }  // namespace cf

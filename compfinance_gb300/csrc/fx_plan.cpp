@@ -90,6 +90,7 @@ bool Context::fxReady(Plan& plan)
         f.vol = reinterpret_cast<const FxVol*>(d + oV);
         f.slope = reinterpret_cast<const double*>(d + oS);
         f.step = reinterpret_cast<const FxStep*>(d + oT);
+        f.node = plan.fxIn.node;
         auto state = [&](double x) {  // the last state not above x
             const double v = std::floor(std::ldexp(x, FX_Y - h.r));
             return !(v > -9.2e18) ? INT64_MIN : v < 9.2e18 ? (long long)v : INT64_MAX;

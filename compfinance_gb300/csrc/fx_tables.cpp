@@ -82,7 +82,8 @@ int lower_with(const FxInput& in, double reach, int r, FxHost& h)
             o[lo] = FxVol{(long long)at, bl, int((b - bl) >> 32)};
             h.slope[size_t(i) * (nS + 1) + lo] = (y[lo] - y[lo - 1]) / (X[lo] - X[lo - 1]) * std::ldexp(1.0, -FX_G);
         }
-        h.step.push_back(FxStep{std::llrint(std::ldexp(in.tw[i], 62)), in.sq[i], in.colA[i], in.colB[i]});
+        h.step.push_back(FxStep{std::llrint(std::ldexp(in.tw[i], 62)), in.sq[i], in.colA[i] * in.node.c,
+                                in.colB[i] * in.node.c, in.colA[i], in.colB[i]});
     }
     return 1;
 }

@@ -10,6 +10,7 @@ namespace cf {
 struct FxInput
 {
     int nSteps = 0;
+    NodeStride node = {1, 1};     // of the reverse's slab
     double x0 = 0;                // log S0
     std::vector<double> X;        // knots, log S - log S0
     std::vector<double> Y;        // [nSteps][X.size()] sqrt(dt) sigma

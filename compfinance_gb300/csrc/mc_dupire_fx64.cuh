@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx6
         }
         head += n;
         __syncthreads();
-        fx_node_flush(p.acc, node, nNodes, RB);
+        fx_node_flush<false>(p, p.acc, node, nNodes, RB);
         __syncthreads();
     };
 

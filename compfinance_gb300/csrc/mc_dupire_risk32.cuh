@@ -70,7 +70,8 @@ __host__ __device__ inline R32Layout r32_layout(int rng, int block, const McPara
     size_t off = 0;
     L.slab = off;
     off += a16(size_t(4 + 2 * p.nPay + 2) * 16);
-    L.node = off;  // int32 local-vol node slab of the current chunk
+    L.node = off;  // int32 local-vol node slab of the current chunk, node (l, c) at c nS + l: the lanes
+                   // of a warp, mostly at one step and so one column, add at different banks
     off += a16(size_t(p.nS) * p.nT * 4);
     L.ir = off;
     off += a16(size_t(p.nS + 1) * 8);
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(RB, RB > 128 ? 4 : (PROD == PROD_UOC && RNGK =
     // shared adds.  gnode is written only by these adds during a sweep and only by its owning
     // thread between sweeps (barriers in between).
     auto bigAdd = [&](const int4 sc, int j, float c) {
-        long long* g = gnode + j * nT;
+        long long* g = gnode + j;
         atomicAdd(reinterpret_cast<unsigned long long*>(g + sc.x),
                   (unsigned long long)__float2ll_rn(c * __int_as_float(sc.z)));
         const float wb = __int_as_float(sc.w);
@@ -511,13 +512,13 @@ __global__ void __launch_bounds__(RB, RB > 128 ? 4 : (PROD == PROD_UOC && RNGK =
                     if (fabsf(av) < AV_MAX)
                     {
                         const float wa = __int_as_float(sc.z), wb = __int_as_float(sc.w);
-                        int* nl = node + jl * nT;
+                        int* nl = node + jl;
                         atomicAdd(nl + sc.x, __float2int_rn(cL * wa));
                         if (wb != 0.0f) atomicAdd(nl + sc.y, __float2int_rn(cL * wb));
                         if (inner && cR != 0.0f)
                         {
-                            atomicAdd(nl + nT + sc.x, __float2int_rn(cR * wa));
-                            if (wb != 0.0f) atomicAdd(nl + nT + sc.y, __float2int_rn(cR * wb));
+                            atomicAdd(nl + sc.x + 1, __float2int_rn(cR * wa));
+                            if (wb != 0.0f) atomicAdd(nl + sc.y + 1, __float2int_rn(cR * wb));
                         }
                     }
                     else
@@ -669,7 +670,8 @@ __global__ void __launch_bounds__(RB, RB > 128 ? 4 : (PROD == PROD_UOC && RNGK =
     // node words in units of 2^-nodeShiftF (nodeShiftF <= FIX_HI_SHIFT): exact in the hi word
     for (int i = tid; i < nNodes; i += RB)
     {
-        const long long v = __ldcg(gnode + i);
+        const int l = i / nT;
+        const long long v = __ldcg(gnode + (i - l * nT) * nS + l);
         if (v) atomicAdd(reinterpret_cast<unsigned long long*>(&p.acc[2 * (1 + i)]),
                          (unsigned long long)(v << (FIX_HI_SHIFT - p.nodeShiftF)));
     }

@@ -86,7 +86,7 @@ __host__ __device__ inline RevLayout rev_layout(const Multi32Args& A)
     RevLayout L;
     size_t off = 0;
     L.node = off;
-    off += a16(size_t(p.nS) * p.nT * 4);
+    off += a16(size_t(node_words(p.nS, p.nT)) * 4);
     L.ir = off;
     off += a16(size_t(p.nS + 1) * 8);
     L.stepc = off;
@@ -393,12 +393,13 @@ __global__ void __launch_bounds__(MB) multi32_reverse(const Multi32Args A)
     long long* spotSlab = reinterpret_cast<long long*>(smem + L.spot);
     int* misc = reinterpret_cast<int*>(smem + L.misc);
     const int tid = threadIdx.x;
-    const int nS = p.nS, nT = p.nT, nSteps = p.nSteps, nNodes = nS * nT, nB = A.nBuckets;
+    const int nS = p.nS, nT = p.nT, nSteps = p.nSteps, nB = A.nBuckets;
+    const NodeStride stride = node_stride(nS, nT);
     const float wScale = ldexpf(1.0f, p.nodeShiftF);
-    for (int i = tid; i < nNodes; i += MB) node[i] = 0;
+    for (int i = tid; i < node_words(nS, nT); i += MB) node[i] = 0;
     for (int i = tid; i < nS + 1; i += MB) sIr[i] = make_float2(p.irF[2 * i], p.irF[2 * i + 1]);
     for (int i = tid; i < nSteps; i += MB)
-        stepc[i] = make_int4(p.colA[i], p.colB[i], __float_as_int(p.cAf[i] * wScale), __float_as_int(p.cBf[i] * wScale));
+        stepc[i] = make_int4(p.colA[i] * stride.c, p.colB[i] * stride.c, __float_as_int(p.cAf[i] * wScale), __float_as_int(p.cBf[i] * wScale));
     if (tid < 2) spotSlab[tid] = 0;
     __syncthreads();
 
@@ -459,24 +460,25 @@ __global__ void __launch_bounds__(MB) multi32_reverse(const Multi32Args A)
                 if (fabsf(av) < AV_MAX)
                 {
                     const float wa = __int_as_float(sc.z), wb = __int_as_float(sc.w);
-                    int* nl = node + jl * nT;
+                    int* nl = node + jl * stride.l;
                     atomicAdd(nl + sc.x, __float2int_rn(cL * wa));
                     if (wb != 0.0f) atomicAdd(nl + sc.y, __float2int_rn(cL * wb));
                     if (inner && cR != 0.0f)
                     {
-                        atomicAdd(nl + nT + sc.x, __float2int_rn(cR * wa));
-                        if (wb != 0.0f) atomicAdd(nl + nT + sc.y, __float2int_rn(cR * wb));
+                        atomicAdd(nl + stride.l + sc.x, __float2int_rn(cR * wa));
+                        if (wb != 0.0f) atomicAdd(nl + stride.l + sc.y, __float2int_rn(cR * wb));
                     }
                 }
                 else
                 {
                     const float ca = __ldg(p.cAf + s), cb = __ldg(p.cBf + s);
-                    fix_add(row + 2 * (1 + jl * nT + sc.x), cL * ca);
-                    if (cb != 0.0f) fix_add(row + 2 * (1 + jl * nT + sc.y), cL * cb);
+                    const int colA = __ldg(p.colA + s), colB = __ldg(p.colB + s);
+                    fix_add(row + 2 * (1 + jl * nT + colA), cL * ca);
+                    if (cb != 0.0f) fix_add(row + 2 * (1 + jl * nT + colB), cL * cb);
                     if (inner && cR != 0.0f)
                     {
-                        fix_add(row + 2 * (1 + (jl + 1) * nT + sc.x), cR * ca);
-                        if (cb != 0.0f) fix_add(row + 2 * (1 + (jl + 1) * nT + sc.y), cR * cb);
+                        fix_add(row + 2 * (1 + (jl + 1) * nT + colA), cR * ca);
+                        if (cb != 0.0f) fix_add(row + 2 * (1 + (jl + 1) * nT + colB), cR * cb);
                     }
                 }
             };
@@ -504,16 +506,20 @@ __global__ void __launch_bounds__(MB) multi32_reverse(const Multi32Args A)
         }
         __syncthreads();
         // the chunk's slab -> the bucket's row (node words in units of 2^-nodeShiftF: exact in hi)
-        for (int i = tid; i < nNodes; i += MB)
-        {
-            const int v = node[i];
+        auto flush = [&](int i, int at) {
+            const int v = node[at];
             if (v)
             {
-                node[i] = 0;
+                node[at] = 0;
                 atomicAdd(reinterpret_cast<unsigned long long*>(row + 2 * (1 + i)),
                           (unsigned long long)((long long)v << hiShift));
             }
-        }
+        };
+        if (stride.c == 1)
+            for (int i = tid; i < nS * nT; i += MB) flush(i, i);
+        else
+            for (int l = tid >> 5; l < nS; l += MW)
+                for (int k = tid & 31; k < nT; k += 32) flush(l * nT + k, k * stride.c + l);
         if (tid == 0)
         {
             fix_flush(row, spotSlab);

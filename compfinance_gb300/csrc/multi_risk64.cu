@@ -58,7 +58,7 @@ __host__ __device__ inline Rev64 rev64_layout(const Multi32Args& A)
         off += (n + 15) & ~size_t(15);
         return o;
     };
-    L.node = take(size_t(A.p.nS) * A.p.nT * 12);
+    L.node = take(size_t(node_words(A.p.nS, A.p.nT)) * 12);
     L.inv = take(size_t(A.p.nS + 1) * 8);
     L.interval = take(size_t(A.p.nS + 1) * 16);
     L.bucket = take(size_t(A.p.fx.nBuckets) * 8);
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(M64_BLOCK, 3) multi64_reverse(const Multi32Arg
     long long* spotSlab = reinterpret_cast<long long*>(smem + L.spot);
     int* misc = reinterpret_cast<int*>(smem + L.misc);
     const int tid = threadIdx.x;
-    const int nS = p.nS, nSteps = p.nSteps, nNodes = nS * p.nT, nB = A.nBuckets, pitch = nS + 1;
+    const int nS = p.nS, nSteps = p.nSteps, nNodes = node_words(nS, p.nT), nB = A.nBuckets, pitch = nS + 1;
     for (int i = tid; i < 3 * nNodes; i += M64_BLOCK) node[i] = 0;
     for (int i = tid; i < nS + 1; i += M64_BLOCK)
     {
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(M64_BLOCK, 3) multi64_reverse(const Multi32Arg
             fix_add_s(spotSlab, ax * 0x1p59 / p.spot);  // x_0 = log(spot)
         }
         __syncthreads();
-        fx_node_flush(row, node, nNodes, M64_BLOCK);
+        fx_node_flush<true>(p, row, node, nNodes, M64_BLOCK);
         if (tid == 0)
         {
             fix_flush(row, spotSlab);

@@ -45,9 +45,11 @@ SERVE_LONG_BLOCKS_PER_SM = 4  # resident blocks per SM of a long request: room f
 # long risks are admitted least work first (a large one queued longer than this goes first)
 SERVE_LONG_ORDER, SERVE_LONG_AGING_MS = 1, 50.0
 SERVE_LOAD_RUNS = 5
-# FP64 form (mc_kernel<double>): ncu of the same kernel at 2^18 paths measures its FP64 pipe 82.9%
-# busy; GB300 executes 2 FP64 FMAs per SM per cycle (ncu's peak of the DFMA counter)
-FP64_PIPE_BUSY_NCU = 0.829
+# FP64 form (dupire_fx64: 64-bit fixed point on the integer pipes): ncu at 2^18 paths measures 232
+# instruction slots (warp instructions x 32) per path-step and the FP64 pipe 21.8% busy; GB300
+# executes 2 FP64 FMAs per SM per cycle (ncu's peak of the DFMA counter)
+INST_PER_PATH_STEP_FP64 = 232.0
+FP64_PIPE_BUSY_NCU = 0.218
 DFMA_PER_SM_PER_CYCLE = 2
 CONFIG = {
     "workload": "dupire_uoc_aad_risk_60x30_156steps_2^22paths_fp32path",
@@ -566,13 +568,16 @@ def main():
         "path_steps_per_s": value * dim,
         "fp64": {"value": world * npath / (t64 / steps64), "unit": "paths/s", "ms_per_step": t64 / steps64 * 1e3,
                  "steps": steps64,
-                 # the same 53 algorithmic flops per path-step against the FP64 FMA peak; the kernel's
-                 # FP64 pipe itself is busier (comparisons, conversions, division/log/exp sequences)
-                 "roofline": {"bound": "fp64_pipe",
+                 # the same 53 algorithmic operations per path-step against the FP64 FMA peak: above 1,
+                 # as the path arithmetic runs in 64-bit fixed point on the integer pipes; its bound
+                 # is instruction issue
+                 "roofline": {"bound": "issue",
                               "achieved": FLOPS_PER_PATH_STEP * steps_tot / (t64 / steps64) / 1e12,
                               "peak": peak_fp64, "unit": "TFLOP/s",
                               "frac": FLOPS_PER_PATH_STEP * steps_tot / (t64 / steps64) / 1e12 / peak_fp64,
                               "fp64_pipe_busy_ncu": FP64_PIPE_BUSY_NCU,
+                              "issue_frac": INST_PER_PATH_STEP_FP64 * steps_tot / (t64 / steps64) /
+                                            (152 * 4 * 32 * sm_max * 1e6),
                               "peak_source": "152 SM x 2 DFMA x 2 x sm_max_mhz of MEASURED_PEAKS.json (the "
                                              "DFMA peak ncu reports; the file measures no FP64 peak)"}},
         "fp32_over_fp64": (t64 / steps64) / per_step,

@@ -10,7 +10,7 @@
 // the unit of a double near log S0 (fx_step), vols 61 fraction bits, Gaussians 59.  Doubles remain where
 // magnitudes range widely: payoffs, exp at maturity, and the reverse's adjoint, whose products with
 // the vol weights are again whole numbers.  Measured (60x30 weekly barrier, mrg32k3a): risk 9.5 ->
-// 0.62 ms at 2^18 paths and 141 -> 5.6 ms at 2^22, value 5.2 -> 0.30 ms at 2^18; 141 instructions per
+// 0.59 ms at 2^18 paths and 141 -> 5.6 ms at 2^22, value 5.2 -> 0.30 ms at 2^18; 141 instructions per
 // path-step of the value run (ncu), issue 58%, ALU pipe 54%, L1 data path 43% of their peaks.
 //
 // Rounds, compaction of the paths with an adjoint and the claimed chunks follow dupire_risk32:

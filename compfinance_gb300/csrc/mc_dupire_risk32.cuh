@@ -100,7 +100,7 @@ __host__ __device__ inline R32Layout r32_layout(int rng, int block, const McPara
 // Sobol barrier variant would spill at 56 registers and keeps eight.  Where shared memory holds fewer
 // blocks (the node slab and the step table of a 120x60 grid with 520 steps leave five), blocks of
 // 256 threads share them: four of those fit, 1024 threads per SM for 640 (200001 paths of that
-// barrier's risk: 1.16 -> 0.86 ms).
+// barrier's risk: 1.16 -> 0.85 ms).
 template <int PROD, int RNGK, bool ROWS, int RB>
 __global__ void __launch_bounds__(RB, RB > 128 ? 4 : (PROD == PROD_UOC && RNGK == RNG_SOBOL) ? 8 : 9)
     dupire_risk32(const McParams p)

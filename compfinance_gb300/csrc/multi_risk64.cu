@@ -6,7 +6,7 @@
 // shared-memory adds and the dependent chain of the adjoint.  The former kernel (multi_kernel.cu,
 // which keeps Black-Scholes and models beyond the fixed-point ranges) ran at the FP64 pipe's and the
 // global 64-bit atomics' rates: each path-step of a maturity cost eight of them.  Measured, 200
-// options on the 60x30 grid, 40 steps, 2^18 Sobol paths: 3.76 -> 1.15 ms (6.8 before its Gaussians
+// options on the 60x30 grid, 40 steps, 2^18 Sobol paths: 3.76 -> 1.12 ms (6.8 before its Gaussians
 // and sums were cheapened).
 #include <cuda_runtime.h>
 

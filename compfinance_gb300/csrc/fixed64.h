@@ -16,8 +16,10 @@
 
 namespace cf {
 
-// The double with bits b as hi 2^-20 + lo 2^-60, rounded to units of 2^-60 (ties to even); false
-// when |v| >= 2^42 (infinities and NaN included), which the caller converts in floating point.
+// The double with bits b as hi 2^-20 + lo 2^-60, rounded to units of 2^-60 (ties to even), with
+// |lo| <= 2^39; false when |v| >= 2^42 (infinities and NaN included), which the caller converts in
+// floating point.  lo has either sign whatever the value's: a sum of low words grows with the root of the
+// number of terms (or, for equal terms, to 2^62 in 2^23 of them), not by 2^39 with each.
 CF_HD bool fix_split_bits(unsigned long long b, long long& hi, long long& lo)
 {
     const int E = int(unsigned(b >> 32) >> 20) & 0x7ff;
@@ -39,6 +41,9 @@ CF_HD bool fix_split_bits(unsigned long long b, long long& hi, long long& lo)
         l = (long long)(m >> -sh);
         l += (rem > half || (rem == half && (l & 1))) ? 1 : 0;
     }
+    const long long carry = (l + (1LL << 39)) >> 40;  // l is below 2^53
+    h += carry;
+    l -= carry << 40;
     const bool neg = (long long)b < 0;
     hi = neg ? -h : h;
     lo = neg ? -l : l;

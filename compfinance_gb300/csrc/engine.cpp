@@ -30,87 +30,6 @@ int launch_gauss(int sobol, int uniform, const unsigned* dir, const unsigned* A,
 
 int fx_node_shift(const Plan& plan, int block);  // fx_plan.cpp
 
-thread_local std::string g_lastError;
-
-int fail(int code, const std::string& msg)
-{
-    g_lastError = msg;
-    return code;
-}
-
-int cuda_fail(cudaError_t e, const char* what)
-{
-    return fail(e == cudaErrorMemoryAllocation ? CF_E_NOMEM : CF_E_CUDA,
-                std::string(what) + ": " + cudaGetErrorString(e));
-}
-
-
-// ------------------------------------------------------------------------------------
-// Device buffers
-// ------------------------------------------------------------------------------------
-std::atomic<unsigned long long> DevBuf::growths{0};
-
-int DevBuf::ensure(size_t n, cudaStream_t stream)
-{
-    if (n <= bytes) return CF_OK;
-    ++growths;
-    const size_t want = n + n / 4;
-    cudaError_t e;
-    if (stream)
-    {
-        // the old buffer is freed after the stream's earlier work, the new one is ready for its later work
-        if (ptr) cudaFreeAsync(ptr, stream);
-        ptr = nullptr;
-        bytes = 0;
-        e = cudaMallocAsync(&ptr, want, stream);
-    }
-    else
-    {
-        release();
-        e = cudaMalloc(&ptr, want);
-    }
-    if (e != cudaSuccess)
-    {
-        ptr = nullptr;
-        bytes = 0;
-        return cuda_fail(e, "cudaMalloc");
-    }
-    bytes = want;
-    return CF_OK;
-}
-
-void DevBuf::release()
-{
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-}
-
-int PinnedBuf::ensure(size_t n)
-{
-    if (n <= bytes) return CF_OK;
-    release();
-    // at least 16 MB (the finished risks of a 200-payoff portfolio on a 120x60 grid are 11.5 MB):
-    // freeing pinned memory waits for the device, so a serving slot should not regrow it
-    const size_t want = std::max(n + n / 4, size_t(16) << 20);
-    cudaError_t e = cudaMallocHost(&ptr, want);
-    if (e != cudaSuccess)
-    {
-        ptr = nullptr;
-        bytes = 0;
-        return cuda_fail(e, "cudaMallocHost");
-    }
-    bytes = want;
-    return CF_OK;
-}
-
-void PinnedBuf::release()
-{
-    if (ptr) cudaFreeHost(ptr);
-    ptr = nullptr;
-    bytes = 0;
-}
-
 Slot::~Slot()
 {
     if (done) cudaEventDestroy(done);
@@ -742,16 +661,15 @@ int Context::init(int dev)
     mrg_jump_tables(A, B);
     int rc = jump.ensure(sizeof(A) + sizeof(B));
     if (rc) return rc;
-    CF_CUDA(cudaMemcpy(jump.ptr, A, sizeof(A), cudaMemcpyHostToDevice));
-    CF_CUDA(cudaMemcpy(static_cast<char*>(jump.ptr) + sizeof(A), B, sizeof(B), cudaMemcpyHostToDevice));
+    if ((rc = jump.upload(A, sizeof(A), stream)) || (rc = jump.upload(B, sizeof(B), stream, sizeof(A)))) return rc;
     jumpA = static_cast<const unsigned*>(jump.ptr);
     jumpB = jumpA + 256 * 12;
     // uniforms: mrg32k3a d / (m1 + 1) (mrg32k3a.h:52,78-79), Sobol s * 2.3283064365387e-10 (sobol.h:26)
     std::vector<float> tab(2 * size_t(INVN_PIECES) * 4);
     inv_normal_table(4294967088.0, tab.data());
     inv_normal_table(1.0 / 2.3283064365387e-10, tab.data() + size_t(INVN_PIECES) * 4);
-    if ((rc = invn.ensure(tab.size() * sizeof(float)))) return rc;
-    CF_CUDA(cudaMemcpy(invn.ptr, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
+    if ((rc = invn.ensure(tab.size() * sizeof(float))) || (rc = invn.upload(tab.data(), tab.size() * sizeof(float), stream)))
+        return rc;
     invnMrg = static_cast<const float*>(invn.ptr);
     invnSobol = invnMrg + size_t(INVN_PIECES) * 4;
     if ((rc = initGauss())) return rc;
@@ -764,26 +682,6 @@ Context::~Context()
     cudaSetDevice(device);
     plans.clear();
     if (ownStream) cudaStreamDestroy(ownStream);
-}
-
-int Context::sobolTables(int dim, McParams& p)
-{
-    DevBuf& b = sobolTabs[dim];
-    if (!b.ptr)
-    {
-        std::vector<uint32_t> t = sobol_dirs(dim);
-        t.resize(size_t(64) * dim, 0u);
-        uint32_t* low = t.data() + size_t(32) * dim;
-        for (int d = 0; d < dim; ++d)
-            for (int l = 1; l < 32; ++l) low[d * 32 + l] = low[d * 32 + l - 1] ^ t[size_t(__builtin_ctz(l)) * dim + d];
-        int rc = b.ensure(t.size() * 4);
-        if (rc) return rc;
-        CF_CUDA(cudaMemcpy(b.ptr, t.data(), t.size() * 4, cudaMemcpyHostToDevice));
-        h2d += t.size() * 4;
-    }
-    p.sobolDir = static_cast<const unsigned*>(b.ptr);
-    p.sobolLow = p.sobolDir + size_t(32) * dim;
-    return CF_OK;
 }
 
 int Context::getPlan(const std::string& mid, const std::string& pid, Plan*& out)

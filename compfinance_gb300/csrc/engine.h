@@ -16,6 +16,7 @@
 
 namespace cf {
 
+extern thread_local std::string g_lastError;
 int fail(int code, const std::string& msg);
 int cuda_fail(cudaError_t e, const char* what);
 // return the failure of a CUDA call as a status (CF_E_CUDA / CF_E_NOMEM with the message)
@@ -38,6 +39,10 @@ struct DevBuf
     // on that stream (no device-wide wait: the buffers of serving slots grow while other slots
     // run)
     int ensure(size_t n, cudaStream_t stream = nullptr);
+    // copies n bytes of pageable host memory to offset `at` and waits for them: kernels on any stream
+    // may read them when this returns (cudaMemcpy may return before its transfer to the device is done, and
+    // the streams here do not wait for the legacy stream)
+    int upload(const void* src, size_t n, cudaStream_t stream, size_t at = 0);
     void release();
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;

@@ -1,5 +1,5 @@
-// Device tables of the FP64 Dupire kernel's fixed-point form (fx_tables.h, mc_dupire_fx64.cuh), built on
-// the first FP64 value or risk run of a (model, product) pair.
+// Device tables of the generators (inverse normals, Sobol), and of the FP64 Dupire kernel's fixed-point form
+// (fx_tables.h, mc_dupire_fx64.cuh), built on the first FP64 value or risk run of a (model, product) pair.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -33,8 +33,31 @@ int Context::initGauss()
     const size_t n = t.g.size() * sizeof(FxgPiece);
     int rc = fxg.ensure(n + sizeof(t.e));
     if (rc) return rc;
-    CF_CUDA(cudaMemcpy(fxg.ptr, t.g.data(), n, cudaMemcpyHostToDevice));
-    CF_CUDA(cudaMemcpy(static_cast<char*>(fxg.ptr) + n, t.e, sizeof(t.e), cudaMemcpyHostToDevice));
+    rc = fxg.upload(t.g.data(), n, stream);
+    return rc ? rc : fxg.upload(t.e, sizeof(t.e), stream, n);
+}
+
+int Context::sobolTables(int dim, McParams& p)
+{
+    DevBuf& b = sobolTabs[dim];
+    if (!b.ptr)
+    {
+        std::vector<uint32_t> t = sobol_dirs(dim);
+        t.resize(size_t(64) * dim, 0u);
+        uint32_t* low = t.data() + size_t(32) * dim;
+        for (int d = 0; d < dim; ++d)
+            for (int l = 1; l < 32; ++l) low[d * 32 + l] = low[d * 32 + l - 1] ^ t[size_t(__builtin_ctz(l)) * dim + d];
+        int rc = b.ensure(t.size() * 4);
+        if (!rc) rc = b.upload(t.data(), t.size() * 4, stream);
+        if (rc)
+        {
+            sobolTabs.erase(dim);  // the next plan of this size starts afresh
+            return rc;
+        }
+        h2d += t.size() * 4;
+    }
+    p.sobolDir = static_cast<const unsigned*>(b.ptr);
+    p.sobolLow = p.sobolDir + size_t(32) * dim;
     return CF_OK;
 }
 

@@ -30,8 +30,6 @@
 
 namespace cf {
 
-extern thread_local std::string g_lastError;
-
 struct Request
 {
     bool generic = false;  // FP64 risk in double arithmetic (smaller scratch)

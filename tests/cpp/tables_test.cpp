@@ -1,0 +1,88 @@
+// Host check of the device tables' uploads against fake_cudart.h: complete when the call returns, whatever
+// stream their readers run on, and made again after a failure.
+#include "fake_cudart.h"
+
+#include <cstdio>
+
+#include "host_math.h"
+
+using namespace cf;
+
+static cudaStream_t const kStream = reinterpret_cast<cudaStream_t>(0x1000);
+
+static int check(const char* what, bool ok)
+{
+    std::printf("%s %s\n", ok ? "ok" : "BAD", what);
+    return !ok;
+}
+
+static bool sobolRight(const McParams& p, int dim)
+{
+    const std::vector<uint32_t> d = sobol_dirs(dim);
+    if (std::memcmp(p.sobolDir, d.data(), size_t(32) * dim * 4)) return false;
+    for (int k = 0; k < dim; ++k)
+        for (int l = 0; l < 32; ++l)
+        {
+            const unsigned g = unsigned(l) ^ (unsigned(l) >> 1);
+            unsigned s = 0;
+            for (int b = 0; b < 5; ++b)
+                if (g >> b & 1) s ^= d[size_t(b) * dim + k];
+            if (p.sobolLow[k * 32 + l] != s) return false;
+        }
+    return true;
+}
+
+static int sobol()
+{
+    int bad = 0;
+    for (int dim : {1, 13, 520})
+    {
+        Context c;
+        c.stream = kStream;
+        McParams p{};
+        bad += check("sobol tables: call", c.sobolTables(dim, p) == CF_OK);
+        bad += check("sobol tables: complete on return", !fake::inFlight() && sobolRight(p, dim));
+        fake::arrive(nullptr);
+    }
+    for (int kind = 0; kind < 2; ++kind)
+    {
+        Context c;
+        c.stream = kStream;
+        McParams p{};
+        (kind ? fake::failCopies : fake::failAllocs) = 1;
+        const size_t held = fake::device.size();
+        bad += check("sobol tables: failure reported", c.sobolTables(13, p) != CF_OK);
+        bad += check("sobol tables: nothing kept after a failure", fake::device.size() == held);
+        bad += check("sobol tables: made again", c.sobolTables(13, p) == CF_OK && !fake::inFlight() && sobolRight(p, 13));
+        fake::arrive(nullptr);
+    }
+    return bad;
+}
+
+static int gauss()
+{
+    Context c;
+    c.stream = kStream;
+    int bad = check("inverse normal tables: call", c.initGauss() == CF_OK);
+    McParams p{};
+    std::vector<FxgPiece> t(FXG_PIECES);
+    bool ok = !fake::inFlight();
+    for (int sobol = 0; sobol < 2; ++sobol)
+    {
+        c.setGenerator(p, sobol != 0);
+        for (int h = 0; h < 2; ++h)
+        {
+            const int g = !sobol ? FXG_MRG : h ? FXG_SOBOL_UPPER : FXG_SOBOL_LOWER;
+            ok = ok && inv_normal_table64(g, t.data()) == p.fx.brk[h] &&
+                 !std::memcmp(t.data(), p.fx.g[h], t.size() * sizeof(t[0]));
+        }
+    }
+    long long e[1 << FX_EXP_BITS];
+    exp_table64(e);
+    ok = ok && !std::memcmp(e, p.fx.expTab, sizeof(e));
+    bad += check("inverse normal and exponential tables: complete on return", ok);
+    fake::arrive(nullptr);
+    return bad;
+}
+
+int main() { return (sobol() + gauss()) != 0; }

@@ -24,6 +24,14 @@ int cuda_fail(cudaError_t e, const char* what)
 
 std::atomic<unsigned long long> DevBuf::growths{0};
 
+// A failed allocation as a status.  The runtime also keeps it as the thread's last error, which would be taken
+// for a failure of the next kernel launch that asks for one: callers may go on with a smaller form.
+static int alloc_fail(cudaError_t e, const char* what)
+{
+    cudaGetLastError();
+    return cuda_fail(e, what);
+}
+
 int DevBuf::ensure(size_t n, cudaStream_t stream)
 {
     if (n <= bytes) return CF_OK;
@@ -47,7 +55,7 @@ int DevBuf::ensure(size_t n, cudaStream_t stream)
     {
         ptr = nullptr;
         bytes = 0;
-        return cuda_fail(e, "cudaMalloc");
+        return alloc_fail(e, "cudaMalloc");
     }
     bytes = want;
     return CF_OK;
@@ -80,7 +88,7 @@ int PinnedBuf::ensure(size_t n)
     {
         ptr = nullptr;
         bytes = 0;
-        return cuda_fail(e, "cudaMallocHost");
+        return alloc_fail(e, "cudaMallocHost");
     }
     bytes = want;
     return CF_OK;

@@ -1,5 +1,5 @@
 // Host check of the device tables' uploads against fake_cudart.h: complete when the call returns, whatever
-// stream their readers run on, and made again after a failure.
+// stream their readers run on, and made again after a failure; buffers that cannot be had.
 #include "fake_cudart.h"
 
 #include <cstdio>
@@ -85,4 +85,23 @@ static int gauss()
     return bad;
 }
 
-int main() { return (sobol() + gauss()) != 0; }
+// A buffer that cannot be had: a status, nothing held, and no error left for the next launch's check.
+static int allocations()
+{
+    int bad = 0;
+    for (int kind = 0; kind < 3; ++kind)
+    {
+        DevBuf d;
+        PinnedBuf h;
+        auto get = [&](size_t n) { return kind == 2 ? h.ensure(n) : d.ensure(n, kind ? kStream : nullptr); };
+        bad += check("buffer: small", get(1000) == CF_OK);
+        fake::failAllocs = 1;
+        bad += check("buffer: out of memory", get(size_t(100) << 20) == CF_E_NOMEM);
+        bad += check("buffer: no error left behind", cudaGetLastError() == cudaSuccess);
+        bad += check("buffer: nothing held", !d.ptr && !d.bytes && !h.ptr && !h.bytes);
+        bad += check("buffer: smaller form", get(2000) == CF_OK);
+    }
+    return bad;
+}
+
+int main() { return (sobol() + gauss() + allocations()) != 0; }

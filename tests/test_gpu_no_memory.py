@@ -1,0 +1,78 @@
+"""FP64 Dupire runs on a device whose memory is taken: the forms with large scratch (records of a
+portfolio's paths, rings of a barrier's rounds) give way to those with little, with the same results, and
+leave no error for the calls after them."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from compfinance_gb300 import Engine
+from compfinance_gb300 import workloads as W
+from gpu_util import num, rel_to_max
+
+pytestmark = pytest.mark.gpu
+
+
+class _Taken:
+    """All but `free` bytes of the device's memory."""
+
+    def __init__(self, free):
+        self.held = []
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        while torch.cuda.mem_get_info()[0] > free + (1 << 28):
+            self.held.append(torch.empty(int(min(torch.cuda.mem_get_info()[0] - free, 32 << 30)), dtype=torch.uint8,
+                                         device="cuda:0"))
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *a):
+        self.held = []
+        torch.cuda.empty_cache()
+
+
+def _put(eng):
+    s, t, v = W.dupire_surface(20, 10)
+    eng.putDupire(100.0, s, t, v, 1.0 / 12.0, "m")
+    eng.putEuropeans([1.0, 1.0, 2.0, 3.0, 3.0], [90.0, 100.0, 110.0, 95.0, 120.0], "book")
+    eng.putBarrier(105.0, 140.0, 3.0, 3.0 / 260, 0.01, 0, "uoc")
+    eng.putBlackScholes(100.0, 0.2, 0, 0.02, 0.01, "bs")
+
+
+def _runs(eng, what):
+    w = np.array([1.0, -0.5, 2.0, 0.25, 1.0])
+    big = num(0, 6000000)  # 3.9 GB of records; the barrier's ring takes 4.3 GB, its smaller form's scratch 1 GB
+    if what == "multi":
+        r = eng.AADriskMulti("m", "book", big)
+        return r["values"], r["risks"]
+    if what == "aggregate":
+        r = eng.AADriskAggregate("m", "book", w, big)
+        return r["payoffValues"], r["risks"]
+    r = eng.AADriskOne("m", "uoc", num(0, 600000))
+    return r["payoffValues"], r["risks"]
+
+
+@pytest.mark.parametrize("what", ["multi", "aggregate", "barrier"])
+def test_gives_way(what):
+    """The two forms differ by a double's rounding of log S per step (2^-51 of it), over sqrt(steps) steps,
+    four deviations; the barrier's band turns it into one of barrier / band width, twice."""
+    eng = Engine(0)
+    try:
+        _put(eng)
+        eng.AADriskMulti("m", "book", num(0, 1000))  # tables and small buffers
+        eng.AADriskOne("m", "uoc", num(0, 1000))
+        with _Taken(3 << 30):
+            taken = _runs(eng, what)
+            # the calls after it check the thread's last error
+            eng.AADriskMulti("bs", "book", num(1, 1000))
+            eng.gaussians(0, 12345, 1234, 4, 0, 10)
+        free = _runs(eng, what)
+        steps = 260 if what == "barrier" else 36
+        tol = 4 * np.sqrt(steps + 1) * np.log(100.0) * 2.0 ** -51
+        band = 140.0 / (2 * 100.0 * 0.01) if what == "barrier" else 1.0
+        assert rel_to_max(taken[0], free[0]) <= tol * band
+        assert rel_to_max(taken[1], free[1]) <= 4 * tol * band
+    finally:
+        eng.close()

@@ -231,6 +231,7 @@ struct Context
     bool multiFast(const Plan& plan) const;
     bool multi32Use(const Plan& plan, const cf_num_param& num) const;  // FP32 Dupire: multi_risk32.cu
     bool multi64Fits(const Plan& plan, const cf_num_param& num) const;  // FP64 Dupire: multi_risk64.cu, if fxReady
+    bool multi64Use(Plan& plan, const cf_num_param& num);  // fits, is ready, and its kernels fit an SM
     size_t multi64Bytes(const Plan& plan, const cf_num_param& num) const;  // its scratch
     // directRisks: the caller's nParam x nPay array, written before the call returns; aggWeights
     // (nPay): the run's risks are those of the weighted sum of the payoffs (nParam values)

@@ -82,7 +82,7 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
     const int nBuckets = slot.evOff[nEv];
     const int nParam = plan.model == MODEL_BS ? 8 : plan.nParam;  // BS: (a, b) per parameter
     const bool fast = multi32Use(plan, num);
-    const bool fx = !fp32 && !generic && multi64Fits(plan, num) && fxReady(plan);
+    const bool fx = !generic && multi64Use(plan, num);
     std::vector<float> ksf(slot.ks.begin(), slot.ks.end());
     std::vector<long long> ksi;  // fixed-point form: the last state at which the spot is not above the strike
     if (fx)
@@ -185,7 +185,8 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
             A.ksI = reinterpret_cast<const long long*>(d + offKsf);
             const size_t recBytes = up(nP * plan.nSteps * 16), evBBytes = up(nE * nP * 2), evSBytes = up(nE * nP * 8);
             rc = slot.scratch.ensure(multi64Bytes(plan, num), st);
-            if (rc == CF_E_NOMEM) return enqueueMulti(slot, plan, num, directRisks, aggWeights, true);
+            // without memory for the records: multi_kernel, or for an aggregate the caller's other form
+            if (rc == CF_E_NOMEM && !aggWeights) return enqueueMulti(slot, plan, num, directRisks, nullptr, true);
             if (rc) return rc;
             char* sc = static_cast<char*>(slot.scratch.ptr);
             A.rec64 = reinterpret_cast<longlong2*>(sc);
@@ -193,9 +194,8 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
             A.evS64 = reinterpret_cast<double*>(sc + recBytes + evBBytes);
             A.list64 = reinterpret_cast<longlong2*>(sc + recBytes + evBBytes + evSBytes);
             const size_t smemF = m64_forward_smem(sobol, A), smemR = m64_reverse_smem(A);
-            rc = smemF > 227 * 1024 || smemR > 227 * 1024 ? 0 : m64_occupancy(sobol, smemF, smemR, &occF, &occR);
+            rc = m64_occupancy(sobol, smemF, smemR, &occF, &occR);
             if (rc) return cuda_fail(cudaError_t(rc), "multi occupancy");
-            if (occF < 1 || occR < 1) return enqueueMulti(slot, plan, num, directRisks, aggWeights, true);
             const long long gridF = std::max(1LL, std::min<long long>((threadsNeeded + 127) / 128, (long long)numSMs * occF));
             rc = launch_multi64(sobol, int(gridF), smemF, numSMs * occR, smemR, A, st);
         }
@@ -296,6 +296,22 @@ bool Context::multi64Fits(const Plan& plan, const cf_num_param& num) const
            (long long)plan.nEv * num.numPath < (1LL << 30) && multi64Bytes(plan, num) <= (size_t(32) << 30);
 }
 
+// And whether its kernels fit an SM: the reverse's slab of nodes, the forward's buckets and strikes.
+bool Context::multi64Use(Plan& plan, const cf_num_param& num)
+{
+    if (!multi64Fits(plan, num) || !fxReady(plan)) return false;
+    Multi32Args A{};
+    A.p = plan.base;
+    A.p.fx = plan.fx;
+    A.nBuckets = plan.nPay + plan.nEv;
+    A.nKs = plan.nPay;
+    const int rng = num.useSobol ? RNG_SOBOL : RNG_MRG;
+    const size_t smemF = m64_forward_smem(rng, A), smemR = m64_reverse_smem(A);
+    int occF = 0, occR = 0;
+    return smemF <= 227 * 1024 && smemR <= 227 * 1024 && !m64_occupancy(rng, smemF, smemR, &occF, &occR) && occF > 0 &&
+           occR > 0;
+}
+
 size_t Context::multi64Bytes(const Plan& plan, const cf_num_param& num) const
 {
     const size_t nP = size_t(num.numPath), nE = size_t(plan.nEv);
@@ -355,13 +371,15 @@ int Context::aggregateRisk(Plan& plan, const cf_num_param& num, const double* we
     // European portfolios on Dupire: the portfolio kernels (every payoff's risks, then their weighted
     // sum on the device) take the work in a fraction of the time of one aggregated adjoint through
     // the generic kernel; the risks are the same linear functional of the paths
-    if (multiFast(plan) && (multi32Use(plan, num) || (multi64Fits(plan, num) && fxReady(plan))))
+    int rc = CF_E_NOMEM;
+    const bool fp32 = multiFast(plan) && multi32Use(plan, num);
+    if (fp32 || (multiFast(plan) && multi64Use(plan, num)))
     {
-        int rc = enqueueMulti(main, plan, num, nullptr, weights);
-        if (rc) return rc;
-        return fetch(main, values, nullptr, aggregate, risks);
+        rc = enqueueMulti(main, plan, num, nullptr, weights);
+        // FP64: one aggregated adjoint needs neither the records nor the payoffs' risks
+        if (rc && (fp32 || rc != CF_E_NOMEM)) return rc;
     }
-    int rc = enqueue(main, plan, num, true, weights);
+    if (rc) rc = enqueue(main, plan, num, true, weights);
     if (rc) return rc;
     return fetch(main, values, nullptr, aggregate, risks);
 }

@@ -114,12 +114,8 @@ bool Context::fxReady(Plan& plan)
         f.slope = reinterpret_cast<const double*>(d + oS);
         f.step = reinterpret_cast<const FxStep*>(d + oT);
         f.node = plan.fxIn.node;
-        auto state = [&](double x) {  // the last state not above x
-            const double v = std::floor(std::ldexp(x, FX_Y - h.r));
-            return !(v > -9.2e18) ? INT64_MIN : v < 9.2e18 ? (long long)v : INT64_MAX;
-        };
-        f.yTop = state(plan.fxTop);
-        f.yBand = state(plan.fxBand);
+        f.yTop = fx_state(plan.base.barSmooth, plan.base.x0d, h.r);
+        f.yBand = fx_state(plan.base.minusSmooth, plan.base.x0d, h.r);
         const double w = plan.fxTop - plan.fxBand, top = plan.base.barSmooth / plan.base.twoSmooth;
         if (w >= 0.0 && w < std::ldexp(0.99, -FX_SMOOTH_BITS)) f.bandScale = top * std::ldexp(1.0, -3 - 62);
     }

@@ -5,6 +5,8 @@
 #include <cmath>
 #include <cstdint>
 
+#include "host_math.h"
+
 namespace cf {
 
 namespace {
@@ -113,6 +115,22 @@ bool fx_lower(const FxInput& in, FxHost& h)
     for (int r = 0, got = 0; r <= 4; ++r)
         if ((got = lower_with(in, reach, r, h)) != 0) return got > 0;
     return false;
+}
+
+long long fx_state(double level, double logSpot, int r)
+{
+    if (!(level > 0.0)) return INT64_MIN;
+    if (std::isinf(level)) return INT64_MAX;
+    double hi, lo;
+    log_dd(level, hi, lo);
+    // hi - logSpot as the rounded difference d and its error (Knuth's two-sum)
+    const double d = hi - logSpot, t = d - hi;
+    lo += (hi - (d - t)) - (logSpot + t);
+    const double v = std::ldexp(d, FX_Y - r), w = std::ldexp(lo, FX_Y - r);
+    if (!(v > -9.2e18)) return INT64_MIN;
+    if (!(v < 9.2e18)) return INT64_MAX;
+    const double f = std::floor(v);
+    return (long long)f + (long long)std::floor((v - f) + w);
 }
 
 }  // namespace cf

@@ -35,4 +35,10 @@ struct FxHost
 // more than 4096 buckets, values that are not numbers.
 bool fx_lower(const FxInput& in, FxHost& h);
 
+// The last state with r bits of range whose spot exp(logSpot + y) is not above level (at the ends of the
+// type where none or every state is).  The logarithm is taken to twice a double's precision: a
+// barrier's survival factor multiplies an error of its level by barrier / band width, the same on all paths
+// (60x30 weekly barrier, 2^18 paths: a double's logarithm cost the mean price up to 3.7e-15).
+long long fx_state(double level, double logSpot, int r);
+
 }  // namespace cf

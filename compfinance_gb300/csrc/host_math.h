@@ -55,6 +55,7 @@ void inv_normal_table(double denom, float* out /* [INVN_PIECES][4] */);
 // halves are the same function of the distance from their end; the truncated constant of the Sobol
 // uniforms makes the upper half 1 - c (2^32 - up), not c up.
 enum FxgGenerator : int { FXG_MRG = 0, FXG_SOBOL_LOWER = 1, FXG_SOBOL_UPPER = 2 };
+void log_dd(double x, double& hi, double& lo);  // log x as hi + lo, finite x > 0
 void exp_table64(long long* out /* [2^FX_EXP_BITS] */);  // 2^(i / 128) in units of 2^-61 (fx_exp)
 unsigned inv_normal_table64(int generator, FxgPiece* pieces /* [FXG_PIECES] */);
 

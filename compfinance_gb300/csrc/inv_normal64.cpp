@@ -104,6 +104,13 @@ long long to_fixed(const DD& v, int shift)
 
 }  // namespace
 
+void log_dd(double x, double& hi, double& lo)
+{
+    const DD l = dd_log(DD(x));
+    hi = l.hi;
+    lo = l.lo;
+}
+
 void exp_table64(long long* out)
 {
     // 2^(1/128) by seven square roots of 2 (Newton steps of r - (r^2 - a) / (2 r)), then its powers

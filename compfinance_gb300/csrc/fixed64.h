@@ -32,18 +32,17 @@ CF_HD bool fix_split_bits(unsigned long long b, long long& hi, long long& lo)
     else if (sh >= 0)
     {
         const int r = 40 - sh;
-        h = (long long)(m >> r);
-        l = (long long)((m & ((1ULL << r) - 1)) << sh);
+        h = (long long)((m + (1ULL << (r - 1))) >> r);
+        l = (long long)((m - ((unsigned long long)h << r)) << sh);
     }
     else if (sh >= -54)
     {
         const unsigned long long half = 1ULL << (-sh - 1), rem = m & (2 * half - 1);
         l = (long long)(m >> -sh);
         l += (rem > half || (rem == half && (l & 1))) ? 1 : 0;
+        h = (l + (1LL << 39)) >> 40;  // l is below 2^53
+        l -= h << 40;
     }
-    const long long carry = (l + (1LL << 39)) >> 40;  // l is below 2^53
-    h += carry;
-    l -= carry << 40;
     const bool neg = (long long)b < 0;
     hi = neg ? -h : h;
     lo = neg ? -l : l;

@@ -78,7 +78,7 @@ bool Context::fxReady(Plan& plan)
 {
     if (plan.fxState != 0) return plan.fxState > 0;
     FxHost h;
-    bool ok = fx_lower(plan.fxIn, h);
+    const bool ok = fx_lower(plan.fxIn, h);
     if (ok)
     {
         std::vector<unsigned char> buf;
@@ -91,10 +91,8 @@ bool Context::fxReady(Plan& plan)
         auto vec = [&](const auto& v) { return put(v.data(), v.size() * sizeof(v[0])); };
         const size_t oB = vec(h.bucket), oI = vec(h.interval), oN = vec(h.inv), oV = vec(h.vol), oS = vec(h.slope),
                      oT = vec(h.step);
-        // the upload completes here: kernels on any slot's stream read the tables
-        ok = plan.fxTables.ensure(buf.size()) == CF_OK &&
-             cudaMemcpyAsync(plan.fxTables.ptr, buf.data(), buf.size(), cudaMemcpyHostToDevice, stream) == cudaSuccess &&
-             cudaStreamSynchronize(stream) == cudaSuccess;
+        // without memory for them this run is the generic kernel's, and the next one tries again
+        if (plan.fxTables.ensure(buf.size()) || plan.fxTables.upload(buf.data(), buf.size(), stream)) return false;
         h2d += buf.size();
         const char* d = static_cast<const char*>(plan.fxTables.ptr);
         FxParams& f = plan.fx;

@@ -2,6 +2,7 @@
 // stream their readers run on, and made again after a failure; buffers that cannot be had.
 #include "fake_cudart.h"
 
+#include <cmath>
 #include <cstdio>
 
 #include "host_math.h"
@@ -104,4 +105,45 @@ static int allocations()
     return bad;
 }
 
-int main() { return (sobol() + gauss() + allocations()) != 0; }
+// The fixed-point tables of a plan: a failed upload sends that run to the generic kernel, not all later ones.
+static int fixedPoint()
+{
+    int bad = 0;
+    for (int kind = 0; kind < 3; ++kind)
+    {
+        Context c;
+        c.stream = kStream;
+        Plan plan;
+        plan.fxState = 0;
+        FxInput& in = plan.fxIn;
+        in.nSteps = 2;
+        in.x0 = std::log(100.0);
+        in.X = {-0.5, 0.0, 0.7};
+        in.Y = {0.05, 0.06, 0.07, 0.04, 0.05, 0.06};
+        in.sq = {0.25, 0.25};
+        in.tw = {0.0, 0.5};
+        in.colA = {0, 0};
+        in.colB = {0, 1};
+        FxHost h;
+        bad += check("fixed point: lowered", fx_lower(in, h));
+        if (kind) (kind == 1 ? fake::failAllocs : fake::failCopies) = 1;
+        if (kind) bad += check("fixed point: failure reported", !c.fxReady(plan) && plan.fxState == 0);
+        bad += check("fixed point: built", c.fxReady(plan) && plan.fxState == 1 && !fake::inFlight());
+        bad += check("fixed point: tables", plan.fx.vol && !std::memcmp(plan.fx.vol, h.vol.data(), h.vol.size() * sizeof(h.vol[0])) &&
+                                                !std::memcmp(plan.fx.bucket, h.bucket.data(), h.bucket.size() * 8));
+        bad += check("fixed point: kept", c.fxReady(plan));
+    }
+    Context c;
+    Plan plan;
+    plan.fxState = 0;
+    plan.fxIn.nSteps = 1;
+    plan.fxIn.X = {0.0, 1e-12};  // knots too close
+    plan.fxIn.Y = {0.05, 0.06};
+    plan.fxIn.sq = {0.25};
+    plan.fxIn.tw = {0.0};
+    plan.fxIn.colA = plan.fxIn.colB = {0};
+    bad += check("fixed point: refused for good", !c.fxReady(plan) && plan.fxState == -1 && !c.fxReady(plan));
+    return bad;
+}
+
+int main() { return (sobol() + gauss() + allocations() + fixedPoint()) != 0; }

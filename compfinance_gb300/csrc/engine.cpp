@@ -564,6 +564,8 @@ int Context::buildPlan(const ModelDesc& m, const ProductDesc& pd, Plan& plan)
         P.logBandD = lb - 1e-9;
         plan.fxTop = P.barSmooth > 0 ? std::log(P.barSmooth) - P.x0d : -INFINITY;
         plan.fxBand = lb - P.x0d;
+        // a level that is not a number knocks nothing out: comparisons in doubles say so, states cannot
+        if (std::isnan(P.barSmooth) || std::isnan(P.minusSmooth)) plan.fxState = -1;
         P.logBandF = float(m.kind == MODEL_DUPIRE ? lb - P.x0d - 1e-5 : lb - 1e-5);
     }
 

@@ -146,8 +146,10 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 ? 1 : sizeof(Real) == 4 ? (RN
     auto SA = [&](int a, int e) -> Real& { return scr[size_t(dim + NP * dim + a * nEv + e) * T]; };
 
     // worst performance at date e (the first minimum, as min_element), its asset
-    // FP64 form: a division takes ten times a product there, so the first minimum is found from products
-    // with the references' reciprocals and only its performance is divided; the divisions by a date's
+    // FP64 form: a division takes ten times a product there, so the minimum is found from products with the
+    // references' reciprocals and only its performance is divided.  Products a rounding apart may be equal
+    // quotients (49 (1 / 49) is below 1), of which the first is the minimum: products whose high words
+    // are next to each other, one pair in 2^18, are compared as quotients.  The divisions by a date's
     // numeraire and by constants are products with their reciprocals
     auto over = [](Real a, Real b, Real inv) { return F32 ? a / b : a * inv; };
     auto worstOf = [&](const Real* s, int& wi) {
@@ -160,7 +162,10 @@ __global__ void __launch_bounds__(MD_BLOCK, NA > 4 ? 1 : sizeof(Real) == 4 ? (RN
                 if (a < nA)
                 {
                     const Real q = s[a] * sInv[a];
-                    if (q < w)
+                    bool less = q < w;
+                    if (unsigned(__double2hiint(q)) - unsigned(__double2hiint(w)) + 1u <= 2u)
+                        less = s[a] / sAsset[a] < sw / sAsset[wi];
+                    if (less)
                     {
                         w = q;
                         sw = s[a];

@@ -49,6 +49,14 @@ CF_HD bool fix_split_bits(unsigned long long b, long long& hi, long long& lo)
     return true;
 }
 
+// A 96-bit word n2 2^64 + n1 2^32 + n0 of units of 2^-60 as hi 2^-20 + lo 2^-60, -2^39 <= lo < 2^39: of either
+// sign, as the split of a double, so that the many flushes of a long run do not sum to a low word of 2^63.
+CF_HD void fix_split_slab(unsigned n0, unsigned n1, unsigned n2, long long& hi, long long& lo)
+{
+    lo = (long long)((((unsigned long long)n1 << 32) | n0) << 24) >> 24;  // the low 40 bits, signed
+    hi = ((long long)(((unsigned long long)n2 << 32) | n1) >> 8) + (lo < 0 ? 1 : 0);
+}
+
 // c + a b / 2^64, rounded.  The low words enter as signed halves, so their product, at most a
 // quarter of the unit, is left out without a bias (error below 0.76 units).  |a|, |b| < 2^62.99.
 // half: the rounding constant, 1/2 in units of 2^-32 of the result's unit.

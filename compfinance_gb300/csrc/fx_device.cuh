@@ -98,8 +98,8 @@ __device__ __forceinline__ void fx_node_flush(const McParams& p, long long* acc,
         if (n0 | n1 | n2)
         {
             node[k] = node[k + nNodes] = node[k + 2 * nNodes] = 0;
-            const long long lo = (long long)(((unsigned long long)(n1 & 0xffu) << 32) | n0);  // 40 bits
-            const long long hi = (long long)(((unsigned long long)n2 << 32) | n1) >> 8;
+            long long hi, lo;
+            fix_split_slab(n0, n1, n2, hi, lo);
             long long* at = acc + 2 * (1 + i);
             if (hi) atomicAdd(reinterpret_cast<unsigned long long*>(at), (unsigned long long)hi);
             if (lo) atomicAdd(reinterpret_cast<unsigned long long*>(at + 1), (unsigned long long)lo);

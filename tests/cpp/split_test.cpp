@@ -1,7 +1,8 @@
 // Host check of the split of a double into the accumulators' two words (fixed64.h):
 // * the low word of every accepted value is at most 2^39 in magnitude, the total is rint(v 2^60);
 // * sums of many terms of one sign in two 64-bit words that wrap around: small and ordinary values,
-//   equal and random ones.
+//   equal and random ones;
+// * the split of a node slab's 96-bit word, likewise.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -62,11 +63,37 @@ static int sum(const char* what, long n, V&& v)
     return !ok;
 }
 
+// Words of a node slab: the low part is at most 2^39, the total is the word; and the flushes of a run of
+// 2^31 paths in sweeps of 128, each of a random positive total, stay in two 64-bit words.
+static int slab()
+{
+    std::mt19937_64 g(8);
+    long bad = 0;
+    __int128 exact = 0;
+    unsigned long long H = 0, L = 0;
+    for (long i = 0; i < (3L << 23); ++i)
+    {
+        __int128 v = (__int128)(g() >> (i & 15));
+        if (i & 1) v = (v << 20) ^ g();
+        const bool neg = i >= (1L << 24) && (i & 2);
+        if (neg) v = -v;
+        long long hi, lo;
+        cf::fix_split_slab((unsigned)v, (unsigned)(unsigned long long)(v >> 32), (unsigned)(unsigned long long)(v >> 64), hi, lo);
+        if (lo < -(1LL << 39) || lo >= (1LL << 39) || ((__int128)hi << 40) + lo != v) ++bad;
+        H += (unsigned long long)hi;
+        L += (unsigned long long)lo;
+        exact += v;
+    }
+    const bool ok = !bad && ((__int128)(long long)H << 40) + (long long)L == exact;
+    std::printf("%s slab words\n", ok ? "ok" : "BAD");
+    return !ok;
+}
+
 int main()
 {
     std::mt19937_64 g(5);
     std::uniform_real_distribution<double> one(0.5, 1.5), small(0.0, 1.0 / 256.0);
-    int bad = words();
+    int bad = words() + slab();
     for (double s : {1.0, -1.0})
     {
         bad += sum("0.003", 300000, [&](long) { return s * 0.003; });

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <vector>
 
 #include "engine.h"
@@ -10,8 +11,8 @@
 
 namespace cf {
 
-// The generators' inverse normal tables and the exponential's, made once per process (20 ms of host
-// work for each of the former).
+// The generators' inverse normal tables and the exponential's, made once per process (20 ms of host work for
+// each of the former, on several cores).
 namespace {
 struct Tables
 {
@@ -20,8 +21,12 @@ struct Tables
     long long e[1 << FX_EXP_BITS];
     Tables() : g(size_t(3) * FXG_PIECES)
     {
-        for (int k = 0; k < 3; ++k) brk[k] = inv_normal_table64(k, &g[size_t(k) * FXG_PIECES]);
+        auto make = [this](int k) { brk[k] = inv_normal_table64(k, &g[size_t(k) * FXG_PIECES]); };
+        auto a = std::async(make, 0), b = std::async(make, 1);  // in this thread where no other can be had
+        make(2);
         exp_table64(e);
+        a.get();
+        b.get();
     }
 };
 }  // namespace

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <future>
 
 #include "host_math.h"
 
@@ -169,7 +170,6 @@ unsigned inv_normal_table64(int gen, FxgPiece* out)
     std::vector<DD> logMant(size_t(nSub) * N);  // log of 1 + (sub + z) / nSub, the same in every binade
     for (int sub = 0; sub < nSub; ++sub)
         for (int j = 0; j < N; ++j) logMant[size_t(sub) * N + j] = dd_log(DD(1.0) + (DD(sub) + DD(z[j])) * DD(1.0 / nSub));
-    bool ok = true;
     auto value = [&](int b, int sub, int j, bool mid) {  // at node j of the piece; j < 0: at its start
         DD up = DD(1.0) + (DD(sub) + DD(j < 0 ? 0.0 : z[j])) * DD(1.0 / nSub);
         up = DD(std::ldexp(up.hi, b), std::ldexp(up.lo, b));
@@ -182,7 +182,7 @@ unsigned inv_normal_table64(int gen, FxgPiece* out)
         }
         return tail(lg);
     };
-    auto fit = [&](int b, int sub, bool mid) {
+    auto fit = [&](int b, int sub, bool mid, bool& ok) {
         FxgPiece r{0, 0, 0, 0, 0};
         if (b <= FXG_SUB_BITS || b == 31)  // one draw at the piece's start, or none
         {
@@ -212,12 +212,22 @@ unsigned inv_normal_table64(int gen, FxgPiece* out)
     };
     const int bBrk = 31 - __builtin_clz(brk);
     const int pBrk = (bBrk << FXG_SUB_BITS) + int(((brk << (31 - bBrk)) >> (31 - FXG_SUB_BITS)) & unsigned(nSub - 1));
-    for (int p = 0; p < FXG_PIECES - 1; ++p)
-    {
-        const int b = p >> FXG_SUB_BITS, sub = p & (nSub - 1);
-        if (p <= pBrk) out[p] = fit(b, sub, false);
-        if (p >= pBrk) out[p + 1] = fit(b, sub, true);
-    }
+    // every piece is on its own: four threads, or this one where no other can be had
+    constexpr int PARTS = 4;
+    auto part = [&](int first) {
+        bool ok = true;
+        for (int p = first; p < FXG_PIECES - 1; p += PARTS)
+        {
+            const int b = p >> FXG_SUB_BITS, sub = p & (nSub - 1);
+            if (p <= pBrk) out[p] = fit(b, sub, false, ok);
+            if (p >= pBrk) out[p + 1] = fit(b, sub, true, ok);
+        }
+        return ok;
+    };
+    std::future<bool> others[PARTS - 1];
+    for (int k = 1; k < PARTS; ++k) others[k - 1] = std::async(part, k);
+    bool ok = part(0);
+    for (std::future<bool>& f : others) ok = f.get() && ok;
     return ok ? brk : 0;
 }
 

@@ -2,8 +2,11 @@
 // stream their readers run on, and made again after a failure; buffers that cannot be had.
 #include "fake_cudart.h"
 
+#include <chrono>
 #include <cmath>
 #include <cstdio>
+#include <ctime>
+#include <thread>
 
 #include "host_math.h"
 
@@ -146,4 +149,23 @@ static int fixedPoint()
     return bad;
 }
 
-int main() { return (sobol() + gauss() + allocations() + fixedPoint()) != 0; }
+// The first context of a process makes the inverse normal tables: on several cores, not one after the other.
+static int firstContext()
+{
+    if (std::thread::hardware_concurrency() < 4) return check("first context: too few cores to tell", true);
+    const auto t0 = std::chrono::steady_clock::now();
+    const std::clock_t c0 = std::clock();  // of all threads
+    Context c;
+    c.stream = kStream;
+    const int bad = check("first context: call", c.initGauss() == CF_OK);
+    const double wall = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() * 1e3;
+    const double cpu = double(std::clock() - c0) / CLOCKS_PER_SEC * 1e3;
+    std::printf("%s first context: %.1f ms for %.1f ms of work\n", wall < 0.6 * cpu ? "ok" : "BAD", wall, cpu);
+    return bad + !(wall < 0.6 * cpu);
+}
+
+int main()
+{
+    const int bad = firstContext();
+    return bad + sobol() + gauss() + allocations() + fixedPoint() != 0;
+}

@@ -816,7 +816,7 @@ int Context::enqueue(Slot& slot, Plan& plan, const cf_num_param& num, bool risk,
             mc_smem_bytes(l, p, 0, &smem0);
             rc = mc_occupancy(l, smem0, &occ0);
             if (rc) return cuda_fail(cudaError_t(rc), "occupancy");
-            p.fx.nodeShift = fx_node_shift(plan, l.block);
+            p.fx.nodeShift = fx_node_shift(plan, 384);  // of every block size: shards may run either
         }
         else
         {

@@ -128,7 +128,8 @@ bool Context::fxReady(Plan& plan)
 }
 
 // Range of a risk launch's vol adjoints: a slab word of 96 bits takes at most `block` paths x (steps that
-// share its time column) of them, each below 2^53 units of 2^-(60 - nodeShift).
+// share its time column) of them, each below 2^53 units of 2^-(60 - nodeShift).  It must not depend on the
+// run's size: larger adjoints are split in doubles, and round differently.
 int fx_node_shift(const Plan& plan, int block)
 {
     int s = 30;

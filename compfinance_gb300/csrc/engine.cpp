@@ -1035,6 +1035,9 @@ void results_from_acc(const long long* acc, int nRisk, int nPay, long long nPath
 
 double fix_value_host(long long hi, long long lo)
 {
+    // one pair of words for each total, so that the value does not depend on how the blocks' carries fell
+    hi += lo >> (FIX_LO_SHIFT - FIX_HI_SHIFT);
+    lo &= (1LL << (FIX_LO_SHIFT - FIX_HI_SHIFT)) - 1;
     return (double)hi * (1.0 / 1048576.0) + (double)lo * (1.0 / 1152921504606846976.0);
 }
 

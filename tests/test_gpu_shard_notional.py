@@ -5,6 +5,7 @@ import pytest
 
 from compfinance_gb300 import Engine, NumericalParam
 from compfinance_gb300 import workloads as W
+from compfinance_gb300.api import results_from_raw
 from compfinance_gb300.shard import shard_range
 
 pytestmark = pytest.mark.gpu
@@ -28,11 +29,11 @@ def test_shards_of_a_large_notional(prod, notional):
             eng.putBarrier(105.0, 150.0, 3.0, 3.0 / 520, 0.01, 0, "p")
         else:
             eng.putEuropean(100.0, 3.0, 3.0, "p")
-        npay, _, _ = eng.shapes("m", "p")
+        npay, npar, _ = eng.shapes("m", "p")
         w = np.full(npay, notional)
         n = 100000
         eng.enqueue("m", "p", NumericalParam(numPath=n, precision="fp64"), risk=True, weights=w)
-        full = _totals(eng.fetch_raw())
+        full, values = _totals(eng.fetch_raw()), eng.fetch(npay, npar)
         total = None
         for k in range(4):
             first, count = shard_range(n, k, 4)
@@ -40,5 +41,7 @@ def test_shards_of_a_large_notional(prod, notional):
             acc = eng.fetch_raw()
             total = acc if total is None else total + acc
         assert _totals(total) == full and any(full)
+        got = results_from_raw(total, npar, npay, n)  # sums beyond 2^33 among them: more than a double's bits
+        assert np.array_equal(got[0], values[0]) and got[2] == values[2] and np.array_equal(got[3], values[3])
     finally:
         eng.close()

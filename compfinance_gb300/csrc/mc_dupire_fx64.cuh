@@ -59,8 +59,9 @@ __host__ __device__ inline FxLayout fx_layout(int rng, int block, const McParams
     return L;
 }
 
-// Resident blocks asked of the compiler: 7 x 128 or 2 x 384 threads (72 and 80 registers) for risk.  The
-// large block shares the slab of a 120 x 60 grid (86 KB), of which two fit an SM.
+// Resident blocks asked of the compiler: 7 x 128 or 2 x 384 threads (72 and 80 registers) for risk; at 72 the
+// barrier spills 44 bytes with mrg32k3a and 24 with Sobol, the European 28 with mrg32k3a.  The large block
+// shares the slab of a 120 x 60 grid (86 KB), of which two fit an SM.
 template <int PROD, int RNGK, bool RISK, int RB>
 __global__ void __launch_bounds__(RB, RISK ? (RB == 128 ? 7 : 2) : 8) dupire_fx64(const McParams p)
 {

@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(FB, 8) multi64_forward(const Multi32Args A)
         if (hist[i]) atomicAdd(A.cnt + i, hist[i]);
 }
 
-// Three blocks of 256 threads per SM (80 registers): the 60x30 grid's slab takes 22 KB, the 120x60
-// grid's 86 KB (two blocks).
+// At least three blocks of 256 threads per SM asked of the compiler, which uses 64 registers: four fit.  The
+// 60x30 grid's slab takes 22 KB, the 120x60 grid's 86 KB (two blocks).
 __global__ void __launch_bounds__(M64_BLOCK, 3) multi64_reverse(const Multi32Args A)
 {
     const McParams& p = A.p;

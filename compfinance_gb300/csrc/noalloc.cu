@@ -148,7 +148,9 @@ extern "C" int cf_aad_risk_aggregate_noalloc(cf_context* ctx, const char* modelI
     size_t smem = 0;
     p.stageY = 0;
     int occ = 0;
-    // the kernel choice of the allocating entry point (cf_aad_risk_aggregate)
+    // FP32: the kernel choice of the allocating entry point (cf_aad_risk_aggregate), in blocks of 128 threads.
+    // FP64 runs the generic kernel, whose scratch is a third of the fixed-point kernel's ring of rounds, and is
+    // an order of magnitude slower than that entry point on Dupire models.
     l.fast = mc_use_fast32(p, plan->prod, l.fp32, 1);
     if (l.fast)
     {

@@ -117,8 +117,9 @@ bool Context::fxReady(Plan& plan)
         f.slope = reinterpret_cast<const double*>(d + oS);
         f.step = reinterpret_cast<const FxStep*>(d + oT);
         f.node = plan.fxIn.node;
-        f.yTop = fx_state(plan.base.barSmooth, plan.base.x0d, h.r);
-        f.yBand = fx_state(plan.base.minusSmooth, plan.base.x0d, h.r);
+        const double x0 = plan.base.x0d, spot = std::exp(x0);
+        f.yTop = fx_today(plan.base.barSmooth, spot, fx_state(plan.base.barSmooth, x0, h.r));
+        f.yBand = fx_today(plan.base.minusSmooth, spot, fx_state(plan.base.minusSmooth, x0, h.r));
         const double w = plan.fxTop - plan.fxBand, top = plan.base.barSmooth / plan.base.twoSmooth;
         if (w >= 0.0 && w < std::ldexp(0.99, -FX_SMOOTH_BITS)) f.bandScale = top * std::ldexp(1.0, -3 - 62);
     }

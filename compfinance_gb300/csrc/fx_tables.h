@@ -41,4 +41,12 @@ bool fx_lower(const FxInput& in, FxHost& h);
 // (60x30 weekly barrier, 2^18 paths: a double's logarithm cost the mean price up to 3.7e-15).
 long long fx_state(double level, double logSpot, int r);
 
+// The same with today's state (0), which all paths share at a product's first date and every state of a model
+// without vol is, above the level when today's spot as a double is: on a level that is today's spot, a
+// payoff's or barrier's slope is one side's or the other's for all of them.
+inline long long fx_today(double level, double spot, long long state)
+{
+    return spot > level ? (state < 0 ? state : -1) : (state > 0 ? state : 0);
+}
+
 }  // namespace cf

@@ -85,11 +85,12 @@ int Context::enqueueMulti(Slot& slot, Plan& plan, const cf_num_param& num, doubl
     const bool fx = !generic && multi64Use(plan, num);
     std::vector<float> ksf(slot.ks.begin(), slot.ks.end());
     std::vector<long long> ksi;  // fixed-point form: the last state at which the spot is not above the strike
+    const double spot = std::exp(plan.base.x0d);
     if (fx)
         for (double k : slot.ks)
         {
             const double x = k > 0.0 ? std::floor(std::ldexp(std::log(k) - plan.base.x0d, FX_Y - plan.fx.r)) : -INFINITY;
-            ksi.push_back(!(x > -9.2e18) ? INT64_MIN : x < 9.2e18 ? (long long)x : INT64_MAX);
+            ksi.push_back(fx_today(k, spot, !(x > -9.2e18) ? INT64_MIN : x < 9.2e18 ? (long long)x : INT64_MAX));
         }
     // device buffer: inputs (bucket offsets, strikes, payoff index per sorted strike), the
     // zeroed accumulators and counters, the bucket segments of the FP32 kernels, the risks

@@ -1,11 +1,10 @@
-"""FP64 Dupire runs on a device whose memory is taken: the forms with large scratch (records of a
+"""FP64 Dupire runs that cannot have the memory they want: the forms with large scratch (records of a
 portfolio's paths, rings of a barrier's rounds) give way to those with little, with the same results, and
-leave no error for the calls after them."""
+leave no error for the calls after them.  The device's memory pool is replaced by one of a few GB."""
 import ctypes
 
 import numpy as np
 import pytest
-import torch
 
 from compfinance_gb300 import Engine
 from compfinance_gb300 import workloads as W
@@ -14,27 +13,29 @@ from gpu_util import num, rel_to_max
 pytestmark = pytest.mark.gpu
 
 
-class _Taken:
-    """All but `free` bytes of the device's memory."""
+class _PoolProps(ctypes.Structure):  # CUmemPoolProps
+    _fields_ = [("allocType", ctypes.c_int), ("handleTypes", ctypes.c_int), ("locationType", ctypes.c_int),
+                ("locationId", ctypes.c_int), ("security", ctypes.c_void_p), ("maxSize", ctypes.c_size_t),
+                ("reserved", ctypes.c_ubyte * 56)]
 
-    def __init__(self, free):
-        self.held = []
-        torch.cuda.synchronize()
-        # what earlier engines gave back to the device's memory pool
-        cu, pool = ctypes.CDLL("libcuda.so.1"), ctypes.c_void_p()
-        assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
-        assert cu.cuMemPoolTrimTo(pool, ctypes.c_size_t(0)) == 0
-        torch.cuda.empty_cache()
-        while torch.cuda.mem_get_info()[0] > free + (1 << 28):
-            self.held.append(torch.empty(int(min(torch.cuda.mem_get_info()[0] - free, 32 << 30)), dtype=torch.uint8,
-                                         device="cuda:0"))
+
+class _SmallPool:
+    """Stream-ordered allocations come from a pool of `size` bytes."""
+
+    def __init__(self, size):
+        self.size, self.cu = size, ctypes.CDLL("libcuda.so.1")
 
     def __enter__(self):
+        self.old, self.pool = ctypes.c_void_p(), ctypes.c_void_p()
+        props = _PoolProps(allocType=1, locationType=1, locationId=0, maxSize=self.size)  # pinned, on the device
+        assert self.cu.cuDeviceGetMemPool(ctypes.byref(self.old), 0) == 0
+        assert self.cu.cuMemPoolCreate(ctypes.byref(self.pool), ctypes.byref(props)) == 0
+        assert self.cu.cuDeviceSetMemPool(0, self.pool) == 0
         return self
 
     def __exit__(self, *a):
-        self.held = []
-        torch.cuda.empty_cache()
+        assert self.cu.cuDeviceSetMemPool(0, self.old) == 0
+        assert self.cu.cuMemPoolDestroy(self.pool) == 0  # its allocations stay valid until they are freed
 
 
 def _put(eng):
@@ -67,12 +68,13 @@ def test_gives_way(what):
         _put(eng)
         eng.AADriskMulti("m", "book", num(0, 1000))  # tables and small buffers
         eng.AADriskOne("m", "uoc", num(0, 1000))
-        with _Taken(3 << 30):
+        with _SmallPool(4 << 30):
             taken = _runs(eng, what)
             # the calls after it check the thread's last error
             eng.AADriskMulti("bs", "book", num(1, 1000))
             eng.gaussians(0, 12345, 1234, 4, 0, 10)
         free = _runs(eng, what)
+        assert not np.array_equal(taken[1], free[1])  # not the same form
         steps = 260 if what == "barrier" else 36
         tol = 4 * np.sqrt(steps + 1) * np.log(100.0) * 2.0 ** -51
         band = 140.0 / (2 * 100.0 * 0.01) if what == "barrier" else 1.0
@@ -92,9 +94,10 @@ def test_aggregate_of_a_large_book():
         eng.putEuropeans([3.0] * 3500, list(np.linspace(60.0, 150.0, 3500)), "book")
         w = np.linspace(0.5, 1.5, 3500) / 3500
         eng.AADriskAggregate("m", "book", w, num(0, 1000))
-        with _Taken(1 << 30):
+        with _SmallPool(1 << 30):
             taken = eng.AADriskAggregate("m", "book", w, num(0, 2000000))  # 1.3 GB of records
         free = eng.AADriskAggregate("m", "book", w, num(0, 2000000))
+        assert not np.array_equal(taken["risks"], free["risks"])
         tol = 4 * np.sqrt(37) * np.log(100.0) * 2.0 ** -51
         assert rel_to_max(taken["payoffValues"], free["payoffValues"]) <= tol
         assert rel_to_max(taken["risks"], free["risks"]) <= 4 * tol

@@ -16,45 +16,78 @@
 
 namespace cf {
 
-// The double with bits b as hi 2^-20 + lo 2^-60, rounded to units of 2^-60 (ties to even), with
-// |lo| <= 2^39; false when |v| >= 2^42 (infinities and NaN included), which the caller converts in
-// floating point.  lo has either sign whatever the value's: a sum of low words grows with the root of the
-// number of terms (or, for equal terms, to 2^62 in 2^23 of them), not by 2^39 with each.
-CF_HD bool fix_split_bits(unsigned long long b, long long& hi, long long& lo)
+// Upper word of the double word (hi, lo) shifted left, lower word of it shifted right, by 0 <= s < 32.
+CF_HD unsigned funnel_left(unsigned lo, unsigned hi, int s)
 {
-    const int E = int(unsigned(b >> 32) >> 20) & 0x7ff;
-    if (E >= 1023 + 42) return false;
-    const unsigned long long m = (b & 0xfffffffffffffULL) | (E ? 0x10000000000000ULL : 0ULL);
-    const int sh = E - 1015;  // |v| 2^60 = m 2^sh
-    long long h = 0, l = 0;
-    if (sh >= 40)
-        h = (long long)(m << (sh - 40));
-    else if (sh >= 0)
-    {
-        const int r = 40 - sh;
-        h = (long long)((m + (1ULL << (r - 1))) >> r);
-        l = (long long)((m - ((unsigned long long)h << r)) << sh);
-    }
-    else if (sh >= -54)
-    {
-        const unsigned long long half = 1ULL << (-sh - 1), rem = m & (2 * half - 1);
-        l = (long long)(m >> -sh);
-        l += (rem > half || (rem == half && (l & 1))) ? 1 : 0;
-        h = (l + (1LL << 39)) >> 40;  // l is below 2^53
-        l -= h << 40;
-    }
-    const bool neg = (long long)b < 0;
-    hi = neg ? -h : h;
-    lo = neg ? -l : l;
-    return true;
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(lo, hi, s);
+#else
+    return (unsigned)(((((unsigned long long)hi << 32) | lo) << s) >> 32);
+#endif
+}
+CF_HD unsigned funnel_right(unsigned lo, unsigned hi, int s)
+{
+#ifdef __CUDA_ARCH__
+    return __funnelshift_r(lo, hi, s);
+#else
+    return (unsigned)((((unsigned long long)hi << 32) | lo) >> s);
+#endif
 }
 
 // A 96-bit word n2 2^64 + n1 2^32 + n0 of units of 2^-60 as hi 2^-20 + lo 2^-60, -2^39 <= lo < 2^39: of either
-// sign, as the split of a double, so that the many flushes of a long run do not sum to a low word of 2^63.
+// sign, so that a sum of low words grows with the root of the number of terms (or, for equal terms, to
+// 2^62 in 2^23 of them), not by 2^39 with each.  The value's own low 40 bits have its sign: in one pair
+// of words 2^24 terms of one sign, or flushes of a node slab, added up to 2^63.
 CF_HD void fix_split_slab(unsigned n0, unsigned n1, unsigned n2, long long& hi, long long& lo)
 {
-    lo = (long long)((((unsigned long long)n1 << 32) | n0) << 24) >> 24;  // the low 40 bits, signed
-    hi = ((long long)(((unsigned long long)n2 << 32) | n1) >> 8) + (lo < 0 ? 1 : 0);
+    const int top = (int)(n1 << 24) >> 24;  // bits 32 to 39, signed
+    lo = (long long)(((unsigned long long)(unsigned)top << 32) | n0);
+    hi = ((long long)(((unsigned long long)n2 << 32) | n1) >> 8) + (top < 0 ? 1 : 0);
+}
+
+// The double with bits b as hi 2^-20 + lo 2^-60, rounded to units of 2^-60 (ties to even), |lo| <= 2^39 as
+// above; false when |v| >= 2^42 (infinities and NaN included), which the caller converts in floating
+// point.  The mantissa is shifted in 32-bit words, as 64-bit shifts by a variable are several instructions each:
+// the 60x30 barrier's FP64 risk of 2^18 paths takes 590 us and the four-asset basket's 155, with them 596 and 162.
+CF_HD bool fix_split_bits(unsigned long long b, long long& hi, long long& lo)
+{
+    const unsigned bh = (unsigned)(b >> 32);
+    const int E = (int)(bh >> 20) & 0x7ff;
+    if (E >= 1023 + 42) return false;
+    unsigned m0 = (unsigned)b, m1 = (bh & 0xfffffu) | 0x100000u;
+    int sh = E - 1015;  // |v| 2^60 = (m1 2^32 + m0) 2^sh
+    if (sh < 0)
+    {
+        // below 2^-8: shifted right and rounded (zero and subnormals to zero)
+        unsigned long long l = 0;
+        if (sh >= -54)
+        {
+            const unsigned long long m = ((unsigned long long)m1 << 32) | m0, half = 1ULL << (-sh - 1), rem = m & (2 * half - 1);
+            l = m >> -sh;
+            l += (rem > half || (rem == half && (l & 1))) ? 1 : 0;
+        }
+        m0 = (unsigned)l;
+        m1 = (unsigned)(l >> 32);
+        sh = 0;
+    }
+    const int s = sh & 31;  // sh is below 50
+    unsigned n0 = m0 << s, n1 = funnel_left(m0, m1, s), n2 = funnel_left(m1, 0, s), n3 = 0;
+    if (sh >= 32)
+    {
+        n3 = n2;
+        n2 = n1;
+        n1 = n0;
+        n0 = 0;
+    }
+    const int top = (int)(n1 << 24) >> 24;
+    lo = (long long)(((unsigned long long)(unsigned)top << 32) | n0);
+    hi = (long long)(((unsigned long long)funnel_right(n2, n3, 8) << 32) | funnel_right(n1, n2, 8)) + (top < 0 ? 1 : 0);
+    if ((int)bh < 0)
+    {
+        hi = -hi;
+        lo = -lo;
+    }
+    return true;
 }
 
 // c + a b / 2^64, rounded.  The low words enter as signed halves, so their product, at most a
